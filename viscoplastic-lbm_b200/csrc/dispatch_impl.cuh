@@ -80,15 +80,20 @@ cudaError_t launch_step_st(const StepParams& p, int op, int rheo, bool odd, Laun
 
 template <int Q, int RHEO, int ST>
 cudaError_t macro_t(const MacroParams& mp, bool odd, cudaStream_t s) {
-    const unsigned g = grid_for(mp.s.N, 256);
-    const bool pr = mp.s.pairH > 0;
-    if (odd) {
-        if (pr) k_macro<Q, RHEO, ST, true, true><<<g, 256, 0, s>>>(mp);
-        else k_macro<Q, RHEO, ST, true, false><<<g, 256, 0, s>>>(mp);
-    } else {
-        if (pr) k_macro<Q, RHEO, ST, false, true><<<g, 256, 0, s>>>(mp);
-        else k_macro<Q, RHEO, ST, false, false><<<g, 256, 0, s>>>(mp);
+    if (mp.s.pairH > 0) {
+        const unsigned g = grid_for(mp.s.N / 2, 256);
+        if (mp.s.pairBlk) {
+            if (odd) k_macro2<Q, RHEO, ST, true, true><<<g, 256, 0, s>>>(mp);
+            else k_macro2<Q, RHEO, ST, false, true><<<g, 256, 0, s>>>(mp);
+        } else {
+            if (odd) k_macro2<Q, RHEO, ST, true, false><<<g, 256, 0, s>>>(mp);
+            else k_macro2<Q, RHEO, ST, false, false><<<g, 256, 0, s>>>(mp);
+        }
+        return cudaGetLastError();
     }
+    const unsigned g = grid_for(mp.s.N, 256);
+    if (odd) k_macro<Q, RHEO, ST, true><<<g, 256, 0, s>>>(mp);
+    else k_macro<Q, RHEO, ST, false><<<g, 256, 0, s>>>(mp);
     return cudaGetLastError();
 }
 
@@ -104,15 +109,20 @@ cudaError_t launch_macro_st(const MacroParams& mp, int rheo, bool odd, cudaStrea
 
 template <int Q, int ST>
 cudaError_t get_pops_t(const StepParams& p, bool odd, float* out, cudaStream_t s) {
-    const unsigned g = grid_for(p.N, 256);
-    const bool pr = p.pairH > 0;
-    if (odd) {
-        if (pr) k_get_pops<Q, ST, true, true><<<g, 256, 0, s>>>(p, out);
-        else k_get_pops<Q, ST, true, false><<<g, 256, 0, s>>>(p, out);
-    } else {
-        if (pr) k_get_pops<Q, ST, false, true><<<g, 256, 0, s>>>(p, out);
-        else k_get_pops<Q, ST, false, false><<<g, 256, 0, s>>>(p, out);
+    if (p.pairH > 0) {
+        const unsigned g = grid_for(p.N / 2, 256);
+        if (p.pairBlk) {
+            if (odd) k_get_pops2<Q, ST, true, true><<<g, 256, 0, s>>>(p, out);
+            else k_get_pops2<Q, ST, false, true><<<g, 256, 0, s>>>(p, out);
+        } else {
+            if (odd) k_get_pops2<Q, ST, true, false><<<g, 256, 0, s>>>(p, out);
+            else k_get_pops2<Q, ST, false, false><<<g, 256, 0, s>>>(p, out);
+        }
+        return cudaGetLastError();
     }
+    const unsigned g = grid_for(p.N, 256);
+    if (odd) k_get_pops<Q, ST, true><<<g, 256, 0, s>>>(p, out);
+    else k_get_pops<Q, ST, false><<<g, 256, 0, s>>>(p, out);
     return cudaGetLastError();
 }
 

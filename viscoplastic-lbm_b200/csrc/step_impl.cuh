@@ -860,8 +860,9 @@ __global__ void __launch_bounds__(256, batch_min_blocks<Q>()) k_step_batched(con
     }
 }
 
-// Macroscopics of the current state (what gpuMacrCollisionStream saves).
-template <int Q, int RHEO, int ST, bool ODD, bool PAIRED>
+// Macroscopics of the current state (what gpuMacrCollisionStream saves), natural
+// layout (k_macro2 for the paired ones).
+template <int Q, int RHEO, int ST, bool ODD>
 __global__ void __launch_bounds__(256) k_macro(const MacroParams mp) {
     const StepParams& p = mp.s;
     const unsigned n = blockIdx.x * blockDim.x + threadIdx.x;
@@ -874,7 +875,7 @@ __global__ void __launch_bounds__(256) k_macro(const MacroParams mp) {
     nb.init(x, y, z, p.nx, p.ny, p.nz);
     float f[Q];
     uint8_t cls;
-    gather<Q, ST, ODD, PAIRED>(p, n, nb, x, y, z, f, cls);
+    gather<Q, ST, ODD>(p, n, nb, x, y, z, f, cls);
     float fx = p.fx, fy = p.fy, fz = p.fz;
     if (mp.fibm_const) {
         const size_t N = (size_t)p.N;
@@ -906,8 +907,9 @@ __global__ void __launch_bounds__(256) k_macro(const MacroParams mp) {
     }
 }
 
-// Populations f_i(x,t) after boundary rules, natural [Q][N] float layout.
-template <int Q, int ST, bool ODD, bool PAIRED>
+// Populations f_i(x,t) after boundary rules, natural [Q][N] float layout, of a
+// natural-layout state (k_get_pops2 for the paired ones).
+template <int Q, int ST, bool ODD>
 __global__ void __launch_bounds__(256) k_get_pops(const StepParams p, float* out) {
     const unsigned n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= (unsigned)p.N) return;
@@ -919,7 +921,7 @@ __global__ void __launch_bounds__(256) k_get_pops(const StepParams p, float* out
     nb.init(x, y, z, p.nx, p.ny, p.nz);
     float f[Q];
     uint8_t cls;
-    gather<Q, ST, ODD, PAIRED>(p, n, nb, x, y, z, f, cls);
+    gather<Q, ST, ODD>(p, n, nb, x, y, z, f, cls);
 #pragma unroll
     for (int i = 0; i < Q; ++i) out[(size_t)i * (size_t)p.N + n] = f[i] + Lattice<Q>::w(i) * p.rho0;
 }
@@ -1050,14 +1052,98 @@ struct BlkNbr {
     }
 };
 
-// One thread advances the node pair (x, y, zp) / (x, y, zp+H), pair-node m.
-// Every access is one aligned vector of the two nodes, also for the x-shifted
-// neighbours of the odd step; crossing the periodic z seam swaps the two lanes.
-//
-// BLK (blocked pairs, NX % 32 == 0): a warp's 32 pairs are one block, whose Q
+// A node pair's place in the population array and its neighbours.  BLK
+// (blocked pairs, NX % 32 == 0): a warp's 32 pairs are one block, whose Q
 // planes follow each other, so plane j of the thread's own pair is at a
 // compile-time offset (32 j) from one pointer, and a neighbour's is that plus
 // one of six axis offsets formed once per thread (BlkNbr).
+template <int Q, int ST, bool ODD, bool BLK>
+struct PairNode {
+    using PV = Pair<ST>;
+    using V = typename PV::V;
+    int x, y, zp;
+    unsigned m;
+    size_t Np;                    // pairs per plane (plain pairs)
+    size_t own;                   // first element of the pair's block column (blocked pairs)
+    bool seam_lo, seam_hi;
+    Nbr pn;                       // neighbour offsets in pair space
+    BlkNbr bn;
+    __device__ __forceinline__ void init(const StepParams& p, unsigned m_) {
+        m = m_;
+        x = (int)(m % (unsigned)p.nx);
+        const unsigned t = m / (unsigned)p.nx;
+        y = (int)(t % (unsigned)p.ny);
+        zp = (int)(t / (unsigned)p.ny);
+        pn.init(x, y, zp, p.nx, p.ny, p.pairH);
+        seam_lo = zp == 0;
+        seam_hi = zp == p.pairH - 1;
+        Np = (size_t)p.N >> 1;
+        own = BLK ? (size_t)(m >> 5) * (Q * 32) + (m & 31u) : 0;
+        if (BLK && ODD) bn.template init<Q>(pn, m);
+    }
+    // Populations streamed to the pair, as stored (both nodes per vector).
+    __device__ __forceinline__ void load(const StepParams& p, V (&in)[Q]) const {
+        const V* __restrict__ P = reinterpret_cast<const V*>(p.pop);
+        const V* __restrict__ Pown = P + own;
+#pragma unroll
+        for (int j = 0; j < Q; ++j) {
+            if (BLK) {
+                if (!ODD) {
+                    in[j] = Pown[32 * j];
+                } else {
+                    const int i = lat_opp(j);
+                    in[i] = Pown[(ptrdiff_t)bn.off(-lat_cx(i), -lat_cy(i), -lat_cz(i)) + 32 * j];
+                }
+            } else if (!ODD) {
+                in[j] = P[(size_t)j * Np + m];
+            } else {
+                const int i = lat_opp(j);
+                in[i] = P[(size_t)j * Np + (unsigned)((int)m + pn.off(-lat_cx(i), -lat_cy(i), -lat_cz(i)))];
+            }
+        }
+        // Crossing the z seam exchanges the lanes.  Only the two seam planes of
+        // the pair space do it, and a warp lies in one plane, so one uniform
+        // branch replaces a select per population.
+        if (ODD && (seam_lo || seam_hi)) {
+#pragma unroll
+            for (int i = 1; i < Q; ++i) {
+                const int cz = lat_cz(i);
+                if ((cz > 0 && seam_lo) || (cz < 0 && seam_hi)) in[i] = PV::swap(in[i]);
+            }
+        }
+    }
+};
+
+// The boundary rules of a pair's boundary nodes, per lane on scalars, and their
+// side-store slots (-1: no boundary node).
+template <int Q, int ST>
+__device__ __forceinline__ void pair_boundary(const StepParams& p, int x, int y, int zp, unsigned n0, unsigned n1,
+                                              uint8_t c0, uint8_t c1, float2 (&g)[Q], int& slot0, int& slot1) {
+    constexpr bool SC = Pair<ST>::kScaled;
+#pragma unroll
+    for (int lane = 0; lane < 2; ++lane) {
+        const uint8_t cl = lane ? c1 : c0;
+        if (!(cl & NODE_BC)) continue;
+        const unsigned nl = lane ? n1 : n0;
+        const int zl = zp + lane * p.pairH;
+        const int sl = p.bc_slot[nl];
+        if (lane) slot1 = sl; else slot0 = sl;
+        if (p.apply_bc) {
+            float f[Q];
+#pragma unroll
+            for (int i = 0; i < Q; ++i) f[i] = SC ? lane_of(g[i], lane) * p.inv_scale : lane_of(g[i], lane);
+            Nbr nb;
+            nb.init(x, y, zl, p.nx, p.ny, p.nz);
+            apply_bc<Q>(f, p, sl, x, y, zl, nb, nl);
+#pragma unroll
+            for (int i = 0; i < Q; ++i) set_lane(g[i], lane, SC ? f[i] * p.scale : f[i]);
+        }
+    }
+}
+
+// One thread advances the node pair (x, y, zp) / (x, y, zp+H), pair-node m.
+// Every access is one aligned vector of the two nodes, also for the x-shifted
+// neighbours of the odd step; crossing the periodic z seam swaps the two lanes.
 //
 // BULK: the pair holds no boundary and no unused node, so the boundary
 // rules, the side store and the unused-node path are compiled out (the bulk
@@ -1069,53 +1155,16 @@ template <int Q, int OP, int RHEO, int ST, bool ODD, bool BLK, bool BULK>
 __device__ __forceinline__ void step2_pair(const StepParams& p, const unsigned seed, const unsigned m) {
     using PV = Pair<ST>;
     using V = typename PV::V;
-    const int H = p.pairH;
-    const int x = (int)(m % (unsigned)p.nx);
-    const unsigned t = m / (unsigned)p.nx;
-    const int y = (int)(t % (unsigned)p.ny);
-    const int zp = (int)(t / (unsigned)p.ny);
-    Nbr pn;                       // neighbour offsets in pair space
-    pn.init(x, y, zp, p.nx, p.ny, H);
-    const bool seam_lo = zp == 0, seam_hi = zp == H - 1;
+    PairNode<Q, ST, ODD, BLK> pr;
+    pr.init(p, m);
     // node indices: (x, y, zp) is m, (x, y, zp + H) is m + N/2 (the even bulk
     // step needs neither x, y, zp nor the neighbour offsets)
     const unsigned n0 = m, n1 = m + (unsigned)(p.N >> 1);
     // the Power-Law state of both nodes, loaded with the populations
     const float eta0 = (RHEO == VLBM_POWERLAW) ? p.omega[n0] : 0.f;
     const float eta1 = (RHEO == VLBM_POWERLAW) ? p.omega[n1] : 0.f;
-    const size_t Np = (size_t)p.N >> 1;   // pairs per plane (plain pairs)
     V in[Q];
-    const V* __restrict__ P = reinterpret_cast<const V*>(p.pop);
-    const size_t own = BLK ? (size_t)(m >> 5) * (Q * 32) + (m & 31u) : 0;
-    const V* __restrict__ Pown = P + own;
-    BlkNbr bn;
-    if (BLK && ODD) bn.init<Q>(pn, m);
-#pragma unroll
-    for (int j = 0; j < Q; ++j) {
-        if (BLK) {
-            if (!ODD) {
-                in[j] = Pown[32 * j];
-            } else {
-                const int i = lat_opp(j);
-                in[i] = Pown[(ptrdiff_t)bn.off(-lat_cx(i), -lat_cy(i), -lat_cz(i)) + 32 * j];
-            }
-        } else if (!ODD) {
-            in[j] = P[(size_t)j * Np + m];
-        } else {
-            const int i = lat_opp(j);
-            in[i] = P[(size_t)j * Np + (unsigned)((int)m + pn.off(-lat_cx(i), -lat_cy(i), -lat_cz(i)))];
-        }
-    }
-    // Crossing the z seam exchanges the lanes.  Only the two seam planes of
-    // the pair space do it, and a warp lies in one plane, so one uniform
-    // branch replaces a select per population.
-    if (ODD && (seam_lo || seam_hi)) {
-#pragma unroll
-        for (int i = 1; i < Q; ++i) {
-            const int cz = lat_cz(i);
-            if ((cz > 0 && seam_lo) || (cz < 0 && seam_hi)) in[i] = PV::swap(in[i]);
-        }
-    }
+    pr.load(p, in);
     // both nodes as float2: lane 0 is (x, y, zp), lane 1 (x, y, zp + H).  Half
     // storage is read as stored (deviation * scale); the moment sums are
     // scaled instead, and the boundary rules see scaled-back values.
@@ -1126,27 +1175,7 @@ __device__ __forceinline__ void step2_pair(const StepParams& p, const unsigned s
     const uint8_t c0 = p.cls[n0], c1 = p.cls[n1];
     if (BULK && ((c0 | c1) & (NODE_BC | NODE_UNUSED))) return;   // k_step2's pair
     int slot0 = -1, slot1 = -1;
-    if (!BULK && ((c0 | c1) & NODE_BC)) {   // boundary rules per lane, on scalars
-#pragma unroll
-        for (int lane = 0; lane < 2; ++lane) {
-            const uint8_t cl = lane ? c1 : c0;
-            if (!(cl & NODE_BC)) continue;
-            const unsigned nl = lane ? n1 : n0;
-            const int zl = zp + lane * H;
-            const int sl = p.bc_slot[nl];
-            if (lane) slot1 = sl; else slot0 = sl;
-            if (p.apply_bc) {
-                float f[Q];
-#pragma unroll
-                for (int i = 0; i < Q; ++i) f[i] = SC ? lane_of(g[i], lane) * p.inv_scale : lane_of(g[i], lane);
-                Nbr nb;
-                nb.init(x, y, zl, p.nx, p.ny, p.nz);
-                apply_bc<Q>(f, p, sl, x, y, zl, nb, nl);
-#pragma unroll
-                for (int i = 0; i < Q; ++i) set_lane(g[i], lane, SC ? f[i] * p.scale : f[i]);
-            }
-        }
-    }
+    if (!BULK && ((c0 | c1) & NODE_BC)) pair_boundary<Q, ST>(p, pr.x, pr.y, pr.zp, n0, n1, c0, c1, g, slot0, slot1);
     float2 fx2 = f2(p.fx), fy2 = f2(p.fy), fz2 = f2(p.fz);
     if ((c0 | c1) & NODE_IBM_FORCE) {   // IBM force read and reset (lbm.cu:45-58)
         const size_t N = (size_t)p.N;
@@ -1205,26 +1234,26 @@ __device__ __forceinline__ void step2_pair(const StepParams& p, const unsigned s
         const int i = ODD ? j : lat_opp(j);
         in[i] = PV::pack2(g[i], Lattice<Q>::w(i), p, r0, r1);
     }
-    if (ODD && (seam_lo || seam_hi)) {   // lanes exchanged across the z seam, as for the loads
+    if (ODD && (pr.seam_lo || pr.seam_hi)) {   // lanes exchanged across the z seam, as for the loads
 #pragma unroll
         for (int j = 1; j < Q; ++j) {
             const int cz = lat_cz(j);
-            if ((cz > 0 && seam_hi) || (cz < 0 && seam_lo)) in[j] = PV::swap(in[j]);
+            if ((cz > 0 && pr.seam_hi) || (cz < 0 && pr.seam_lo)) in[j] = PV::swap(in[j]);
         }
     }
-    if (ODD) pn.launder();
-    if (ODD && BLK) bn.launder();
+    if (ODD) pr.pn.launder();
+    if (ODD && BLK) pr.bn.launder();
     V* __restrict__ Po = reinterpret_cast<V*>(p.pop);
-    V* __restrict__ Powo = Po + own;
+    V* __restrict__ Powo = Po + pr.own;
 #pragma unroll
     for (int j = 0; j < Q; ++j) {
         if (BLK) {
             if (!ODD) Powo[32 * j] = in[lat_opp(j)];
-            else Powo[(ptrdiff_t)bn.off(lat_cx(j), lat_cy(j), lat_cz(j)) + 32 * j] = in[j];
+            else Powo[(ptrdiff_t)pr.bn.off(lat_cx(j), lat_cy(j), lat_cz(j)) + 32 * j] = in[j];
         } else if (!ODD) {
-            Po[(size_t)j * Np + m] = in[lat_opp(j)];
+            Po[(size_t)j * pr.Np + m] = in[lat_opp(j)];
         } else {
-            Po[(size_t)j * Np + (unsigned)((int)m + pn.off(lat_cx(j), lat_cy(j), lat_cz(j)))] = in[j];
+            Po[(size_t)j * pr.Np + (unsigned)((int)m + pr.pn.off(lat_cx(j), lat_cy(j), lat_cz(j)))] = in[j];
         }
     }
 }
@@ -1273,6 +1302,83 @@ __global__ void __launch_bounds__(256) k_step2(const StepParams p) {
     const unsigned k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= (unsigned)p.n_special) return;
     step2_pair<Q, OP, RHEO, ST, ODD, BLK, false>(p, seed, (unsigned)p.special_pairs[k]);
+}
+
+// ------------------------------------------- read-outs of paired layouts --
+// Macroscopics and populations of a z-paired state, one thread per node pair
+// with the step's own loads.  Bound by memory: each population vector is read
+// once, as whole lines (a thread per node reads every line twice, for one lane
+// at a time), and addressed from one pointer.  D3Q19 FP16 Bingham at 256^3,
+// rho, u and omega: 0.22 ms (58 B per node, 0.67 of the copy bandwidth)
+// against 0.9 ms by node with pair_elem's index arithmetic per population.
+template <int Q, int RHEO, int ST, bool ODD, bool BLK>
+__global__ void __launch_bounds__(256, 2) k_macro2(const MacroParams mp) {
+    const StepParams& p = mp.s;
+    constexpr bool SC = Pair<ST>::kScaled;
+    const unsigned m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= (unsigned)(p.N >> 1)) return;
+    PairNode<Q, ST, ODD, BLK> pr;
+    pr.init(p, m);
+    const unsigned nn[2] = {m, m + (unsigned)(p.N >> 1)};
+    float2 g[Q];
+    {
+        typename Pair<ST>::V in[Q];
+        pr.load(p, in);
+#pragma unroll
+        for (int i = 0; i < Q; ++i) g[i] = Pair<ST>::raw2(in[i]);
+    }
+    const uint8_t c0 = p.cls[nn[0]], c1 = p.cls[nn[1]];
+    int s0 = -1, s1 = -1;
+    if ((c0 | c1) & NODE_BC) pair_boundary<Q, ST>(p, pr.x, pr.y, pr.zp, nn[0], nn[1], c0, c1, g, s0, s1);
+    constexpr bool NEED_PI = RHEO != VLBM_NEWTONIAN;
+    const float2 fx2 = f2(p.fx), fy2 = f2(p.fy), fz2 = f2(p.fz);
+    const Mom2 mm = moments2<Q, NEED_PI, SC>(g, fx2, fy2, fz2, p.rho0, p.inv_scale);
+    const float2 aux = NEED_PI ? stress_aux2(mm, fx2, fy2, fz2) : f2(0.f);
+#pragma unroll
+    for (int lane = 0; lane < 2; ++lane) {
+        const unsigned n = nn[lane];
+        // an unused node is never updated: the initial macroscopics (lbmInitialization.cu:100-111)
+        const bool unused = (lane ? c1 : c0) & NODE_UNUSED;
+        if (mp.rho) mp.rho[n] = unused ? p.rho0 : lane_of(mm.rho, lane);
+        if (mp.ux) mp.ux[n] = unused ? 0.f : lane_of(mm.ux, lane);
+        if (mp.uy) mp.uy[n] = unused ? 0.f : lane_of(mm.uy, lane);
+        if (mp.uz) mp.uz[n] = unused ? 0.f : lane_of(mm.uz, lane);
+        if (mp.omega_out) {
+            float omega = p.omega_newt;
+            if (RHEO != VLBM_NEWTONIAN) {
+                const float old = (RHEO == VLBM_POWERLAW) ? p.omega[n] : 0.f;
+                float eta = 0.f;
+                omega = relax<RHEO>(p, old, lane_of(aux, lane), eta);
+            }
+            mp.omega_out[n] = unused ? 0.f : omega;
+        }
+    }
+}
+
+template <int Q, int ST, bool ODD, bool BLK>
+__global__ void __launch_bounds__(256, 2) k_get_pops2(const StepParams p, float* out) {
+    constexpr bool SC = Pair<ST>::kScaled;
+    const unsigned m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= (unsigned)(p.N >> 1)) return;
+    PairNode<Q, ST, ODD, BLK> pr;
+    pr.init(p, m);
+    const unsigned n0 = m, n1 = m + (unsigned)(p.N >> 1);
+    float2 g[Q];
+    {
+        typename Pair<ST>::V in[Q];
+        pr.load(p, in);
+#pragma unroll
+        for (int i = 0; i < Q; ++i) g[i] = Pair<ST>::raw2(in[i]);
+    }
+    const uint8_t c0 = p.cls[n0], c1 = p.cls[n1];
+    int s0 = -1, s1 = -1;
+    if ((c0 | c1) & NODE_BC) pair_boundary<Q, ST>(p, pr.x, pr.y, pr.zp, n0, n1, c0, c1, g, s0, s1);
+#pragma unroll
+    for (int i = 0; i < Q; ++i) {
+        const float rest = Lattice<Q>::w(i) * p.rho0;
+        out[(size_t)i * (size_t)p.N + n0] = (SC ? g[i].x * p.inv_scale : g[i].x) + rest;
+        out[(size_t)i * (size_t)p.N + n1] = (SC ? g[i].y * p.inv_scale : g[i].y) + rest;
+    }
 }
 
 }  // namespace vlbm
