@@ -134,3 +134,47 @@ def test_ibm_step_bit_reproducible(vlbm):
         sim.close()
     np.testing.assert_array_equal(out[0][0], out[1][0])
     np.testing.assert_array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("diameter,center,walls", [
+    (1.5, (7.9, 8.2, 8.4), 1),      # few nodes: part-filled groups of lanes, one CTA
+    (3.0, (0.4, 8.1, 15.7), 0),     # stencils across two periodic faces
+    (7.0, (8.3, 3.6, 8.0), 1),      # stencils cut by a wall
+    (9.0, (8.1, 8.0, 7.8), 0),      # several CTAs per sphere, the last one part-filled
+])
+def test_ibm_node_counts_match_oracle(vlbm, oracle, diameter, center, walls):
+    w = dict(wall_x=walls, wall_y=1, wall_z=walls)
+    sim, o, sp = make_case(vlbm, oracle, 19, 3 if walls else 1, (16, 17, 18),
+                           [dict(diameter=diameter, cx=center[0], cy=center[1], cz=center[2], vx=0.01, wz=0.003,
+                                 density=2.0, movable=1)],
+                           dict(max_iterations=2, gx=0.0, gy=0.0, gz=-1e-5, **w), dict(tau=0.8), 0)
+    sim.step(6)
+    o.step(6)
+    pg, po = sim.particles(1)[0], o.particles()
+    assert np.abs(np.array(list(pg.vel)) - po["vel"][0]).max() <= 2e-3 * np.abs(po["vel"]).max()
+    assert np.abs(np.array(list(pg.w)) - po["w"][0]).max() <= 2e-3 * np.abs(po["w"]).max() + 1e-9
+    mg, mo = sim.macroscopics(), o.macroscopics()
+    for k in ("ux", "uy", "uz"):
+        assert np.abs(mg[k] - mo[k]).max() <= 5e-6, k
+
+
+def test_checkpoint_image_keeps_ibm_macroscopics_as_planes(vlbm):
+    cfg = vlbm.Config.default(nx=16, ny=18, nz=20, tau=0.8)
+    sim = vlbm.Simulation(cfg, builder=vlbm.BUILDER_CLOSED_BOX)
+    sim.add_spheres(vlbm.IbmConfig.default(**CLOSED),
+                    [vlbm.Sphere(diameter=6, cx=8, cy=8, cz=9, vx=0.01, density=1.5, movable=1)])
+    sim.step(1)
+    image = sim.checkpoint().tobytes()
+    off = int(np.frombuffer(image, np.uint32, 1, 12)[0])   # header_bytes
+    regions = {}
+    while off < len(image) - 8:
+        rid, _ = np.frombuffer(image, np.uint32, 2, off)
+        size = int(np.frombuffer(image, np.uint64, 1, off + 8)[0])
+        regions[int(rid)] = image[off + 16:off + 16 + size]
+        off += 16 + size
+    planes = np.frombuffer(regions[112], np.float32).reshape(4, 20, 18, 16)
+    box = planes[0] != 0
+    assert 100 < box.sum() < box.size
+    m = sim.macroscopics()
+    for k, name in enumerate(("rho", "ux", "uy", "uz")):
+        np.testing.assert_array_equal(planes[k][box], m[name][box])

@@ -89,6 +89,28 @@ cudaError_t ckpt_copy(vlbm_sim* s, void* dst, const void* src, size_t bytes, cud
     return e == cudaSuccess ? cudaStreamSynchronize(s->stream) : e;
 }
 
+// One region between the device and the image (to_image: out of the device).
+// A region of float4 records goes through planes on the device, so the image
+// does not depend on how the device lays the four values out.
+cudaError_t region_copy(vlbm_sim* s, const StateRegion& r, void* host, bool to_image) {
+    if (!r.records4)
+        return to_image ? ckpt_copy(s, host, r.dev, r.bytes, cudaMemcpyDeviceToHost)
+                        : ckpt_copy(s, r.dev, host, r.bytes, cudaMemcpyHostToDevice);
+    const size_t N = r.bytes / (4 * sizeof(float));
+    void* planes = nullptr;
+    cudaError_t e = cudaMallocAsync(&planes, r.bytes, s->stream);
+    if (e != cudaSuccess) return e;
+    if (to_image) {
+        e = ibm_planes(r.dev, static_cast<float*>(planes), N, true, s->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(host, planes, r.bytes, cudaMemcpyDeviceToHost, s->stream);
+    } else {
+        e = cudaMemcpyAsync(planes, host, r.bytes, cudaMemcpyHostToDevice, s->stream);
+        if (e == cudaSuccess) e = ibm_planes(r.dev, static_cast<float*>(planes), N, false, s->stream);
+    }
+    cudaFreeAsync(planes, s->stream);
+    return e == cudaSuccess ? cudaStreamSynchronize(s->stream) : e;
+}
+
 float effective_scale(const vlbm_sim* s) {
     if (s->cfg.storage_scale > 0) return (float)s->cfg.storage_scale;
     return s->cfg.storage == VLBM_STORE_F16 ? 4096.0f : 1.0f;
@@ -194,7 +216,7 @@ vlbm_status save_image(vlbm_sim* s, std::vector<unsigned char>* grow, void* buf,
         RegionHeader rh{r.id, 0u, (uint64_t)r.bytes};
         std::memcpy(out + off, &rh, sizeof(rh));
         off += sizeof(rh);
-        e = ckpt_copy(s, out + off, r.dev, r.bytes, cudaMemcpyDeviceToHost);
+        e = region_copy(s, r, out + off, true);
         if (e != cudaSuccess) return cuda_status(e, "checkpoint: read device state");
         off += r.bytes;
     }
@@ -257,7 +279,7 @@ vlbm_status load_image(vlbm_sim* s, const unsigned char* in, size_t n) {
     off = sizeof(CkptHeader);
     for (const auto& r : regions) {
         off += sizeof(RegionHeader);
-        cudaError_t e = ckpt_copy(s, r.dev, in + off, r.bytes, cudaMemcpyHostToDevice);
+        cudaError_t e = region_copy(s, r, const_cast<unsigned char*>(in + off), false);
         if (e != cudaSuccess) return cuda_status(e, "checkpoint: write device state");
         off += r.bytes;
     }

@@ -15,12 +15,12 @@
 //   k_ibm_gather     several CTAs per sphere: rho,u of the post-boundary
 //                    populations with the constant body force
 //                    (gpuUpdateMacrIBM ibm.cu:544-648) for the box nodes,
-//                    written to dense fields; each node's owner becomes the
+//                    written as one record per node; each node's owner becomes the
 //                    lowest index of the spheres whose box holds it
 //   per multi-direct-forcing iteration:
-//     k_ibm_interp_spread  several CTAs per sphere, one warp per Lagrangian
-//                    node with its 64 stencil points split over the lanes:
-//                    Peskin 4-point interpolation (warp reduction), direct
+//     k_ibm_interp_spread  several CTAs per sphere, 16 lanes per Lagrangian
+//                    node with its 64 stencil points split over them: Peskin
+//                    4-point interpolation (shuffle reduction), direct
 //                    forcing, spreading with fixed-point atomics; per-CTA
 //                    force/torque partials
 //     k_ibm_update   one warp per sphere: partials added in a fixed order, particle velocity and
@@ -45,8 +45,9 @@ namespace vlbm {
 
 constexpr int IBM_MAX_SLOTS = 13;           // MAX_ACTIVE_COLLISIONS, ibmBoundaryCondition.h:78
 constexpr int IBM_THREADS = 256;
-constexpr int IBM_NODES_PER_CTA = 32;       // Lagrangian nodes per CTA of k_ibm_interp_spread (4 per warp)
-constexpr int IBM_MAX_SPLIT = 32;           // CTAs per sphere, at most
+constexpr int IBM_NODE_LANES = 16;          // lanes per Lagrangian node in the interpolation
+constexpr int IBM_NODES_PER_CTA = 32;       // Lagrangian nodes per CTA of k_ibm_interp_spread (2 per group of lanes)
+constexpr int IBM_MAX_SPLIT = 64;           // CTAs per sphere, at most
 constexpr int IBM_MAX_PARTICLES = 1024;   // pair buffer np*np*6 doubles <= 50 MB
 constexpr unsigned IBM_NO_OWNER = 0xFFFFFFFFu;   // owner[] of a node in no sphere's box
 
@@ -78,7 +79,7 @@ struct IbmState {
     double *nx = nullptr, *ny = nullptr, *nz = nullptr, *nS = nullptr;
     double *nfx = nullptr, *nfy = nullptr, *nfz = nullptr, *ndx = nullptr, *ndy = nullptr, *ndz = nullptr;
     int* npid = nullptr;
-    float* fields = nullptr;      // [4][N] rho,ux,uy,uz (IBM macroscopics)
+    float4* fields = nullptr;     // [N] (rho, ux, uy, uz): IBM macroscopics, one 16-byte record per node
     unsigned long long* faux = nullptr;   // [3][N] spread force, fixed point (IBM_FIX_SCALE)
     unsigned* owner = nullptr;    // [N] lowest sphere index whose box holds the node, during a step;
                                   // IBM_NO_OWNER everywhere between steps
@@ -231,34 +232,34 @@ __device__ __forceinline__ unsigned box_size(const DPart& p) {
 // iteration updates a node once, from that sphere's CTAs, and the last pass
 // sets it back to IBM_NO_OWNER.
 template <int Q, int ST, bool ODD, bool PAIRED>
+__device__ __forceinline__ void gather_box_node(const StepParams& sp, const IbmParams& P, const DPart& p,
+                                                unsigned sphere, unsigned k, float4* fields, unsigned* owner) {
+    const unsigned bx = (unsigned)p.box_n[0], by = (unsigned)p.box_n[1];
+    const unsigned t = k / bx;
+    const int ix = (int)(k - t * bx), iy = (int)(t % by), iz = (int)(t / by);
+    const int x = wrap_box(p.box_lo[0] + ix, P.nx), y = wrap_box(p.box_lo[1] + iy, P.ny),
+              z = wrap_box(p.box_lo[2] + iz, P.nz);
+    const unsigned n = (unsigned)(((size_t)z * P.ny + y) * P.nx + x);
+    Nbr nb;
+    nb.init(x, y, z, sp.nx, sp.ny, sp.nz);
+    float f[Q];
+    uint8_t cls;
+    gather<Q, ST, ODD, PAIRED>(sp, n, nb, x, y, z, f, cls);
+    const Mom m = moments<Q, false>(f, P.fx, P.fy, P.fz, sp.rho0);
+    fields[n] = make_float4(m.rho, m.ux, m.uy, m.uz);
+    atomicMin(&owner[n], sphere);
+}
+
+template <int Q, int ST, bool ODD, bool PAIRED>
 __global__ void __launch_bounds__(IBM_THREADS) k_ibm_gather(StepParams sp, IbmParams P, const DPart* parts,
-                                                             float* fields, unsigned* owner, int split) {
+                                                             float4* fields, unsigned* owner, int split) {
     chain_enter();
     // `split` CTAs per sphere share its box
     const unsigned sphere = blockIdx.x / split;
     const DPart& p = parts[sphere];
-    const int sub = blockIdx.x % split;
-    const unsigned bx = (unsigned)p.box_n[0], by = (unsigned)p.box_n[1];
     const unsigned tot = box_size(p);
-    const size_t N = (size_t)sp.N;
-    for (unsigned k = sub * blockDim.x + threadIdx.x; k < tot; k += split * blockDim.x) {
-        const unsigned t = k / bx;
-        const int ix = (int)(k - t * bx), iy = (int)(t % by), iz = (int)(t / by);
-        const int x = wrap_box(p.box_lo[0] + ix, P.nx), y = wrap_box(p.box_lo[1] + iy, P.ny),
-                  z = wrap_box(p.box_lo[2] + iz, P.nz);
-        const unsigned n = (unsigned)(((size_t)z * P.ny + y) * P.nx + x);
-        Nbr nb;
-        nb.init(x, y, z, sp.nx, sp.ny, sp.nz);
-        float f[Q];
-        uint8_t cls;
-        gather<Q, ST, ODD, PAIRED>(sp, n, nb, x, y, z, f, cls);
-        const Mom m = moments<Q, false>(f, P.fx, P.fy, P.fz, sp.rho0);
-        fields[n] = m.rho;
-        fields[N + n] = m.ux;
-        fields[2 * N + n] = m.uy;
-        fields[3 * N + n] = m.uz;
-        atomicMin(&owner[n], sphere);
-    }
+    for (unsigned k = (blockIdx.x % split) * blockDim.x + threadIdx.x; k < tot; k += split * blockDim.x)
+        gather_box_node<Q, ST, ODD, PAIRED>(sp, P, p, sphere, k, fields, owner);
 }
 
 // ------------------------------------------------------------- contacts --
@@ -571,63 +572,18 @@ __global__ void __launch_bounds__(IBM_THREADS) k_ibm_begin(IbmParams P, DPart* p
 }
 
 // -------------------------------------------------- interpolation/spread --
-// Stencil of one Lagrangian node: base index and validity range per axis.
-struct NodeStencil {
-    int base[3], lo[3], hi[3];
-    float w[3][4];
-    bool skip;
-};
-
-__device__ __forceinline__ NodeStencil node_stencil(const IbmParams& P, const DPart& p, double X, double Y, double Z) {
-    NodeStencil s;
-    const double pos[3] = {X, Y, Z};
-    const double L[3] = {(double)P.nx, (double)P.ny, (double)P.nz};
-    const int Li[3] = {P.nx, P.ny, P.nz};
-    s.skip = false;
-    for (int a = 0; a < 3; ++a) {
-        double xu = P.wall[a] ? pos[a] : p.pos[a] + pdelta(pos[a] - p.pos[a], L[a]);
-        if (!(fabs(xu) < 4.0 * L[a] + 8.0)) {  // non-finite or diverged position: no stencil
-            s.skip = true;
-            xu = 0.0;
-        }
-        // int(x) - P_DIST + 1 of the stored coordinate (ibm.cu:236-240): truncation,
-        // which differs from floor for the negative coordinates a sphere's nodes
-        // have across x=0 before their first movement wraps them; for periodic
-        // axes the base is then shifted into the sphere-centred frame
-        const double raw = s.skip ? 0.0 : pos[a];
-        const int braw = (int)raw - 1;
-        const double fr_raw = raw - (double)braw;
-        if (P.wall[a]) {
-            s.base[a] = braw;
-        } else {
-            const int k = (int)rint((xu - raw) / L[a]);
-            s.base[a] = braw + k * Li[a];
-        }
-        s.lo[a] = 0;
-        s.hi[a] = 3;
-        if (P.wall[a]) {
-            s.hi[a] = (s.base[a] + 3 < Li[a]) ? 3 : (Li[a] - 1 - s.base[a]);
-            s.lo[a] = (s.base[a] >= 0) ? 0 : -s.base[a];
-        }
-        if (s.hi[a] <= 0 || s.lo[a] >= 4) s.skip = true;  // ibm.cu:300-305
-        const float fr = (float)fr_raw;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) s.w[a][j] = stencil4((float)j - fr);
-    }
-    return s;
-}
-
 // Spread force in 2^-48 fixed point, summed with 64-bit integer atomics: the
 // sum does not depend on the order of the additions, so a lattice's IBM step is
 // bit-reproducible from run to run and alone or among other lattices.
 // Resolution 3.6e-15 per contribution (below the FP32 rounding of any
-// contribution above 1e-7), range +-32768 for the sum at one node.
-constexpr double IBM_FIX_SCALE = 281474976710656.0;   // 2^48
+// contribution above 1e-7), range +-32768 for the sum at one node.  Scaling by
+// a power of two is exact in FP32, so the conversion takes the float.
+constexpr float IBM_FIX_SCALE = 281474976710656.0f;   // 2^48
 __device__ __forceinline__ unsigned long long to_fix(float v) {
-    return (unsigned long long)__double2ll_rn((double)v * IBM_FIX_SCALE);
+    return (unsigned long long)__float2ll_rn(v * IBM_FIX_SCALE);
 }
 __device__ __forceinline__ float from_fix(unsigned long long v) {
-    return (float)((double)(long long)v * (1.0 / IBM_FIX_SCALE));
+    return (float)((double)(long long)v * (1.0 / (double)IBM_FIX_SCALE));
 }
 
 // Lattice index of a box-relative offset: the offsets stay within one period
@@ -639,104 +595,173 @@ __device__ __forceinline__ int wrap_near(int v, int n) {
     return v;
 }
 
-// Interpolation, direct forcing and spreading (ibm.cu:307-541).  One warp per
-// Lagrangian node, its 4x4x4 stencil split over the lanes (points q and q+32);
-// a sphere's nodes are shared by IBM_SPLIT CTAs.  The interpolation reads the
-// IBM macroscopic fields and the spreading adds into the auxiliary force field,
-// two different arrays, so each node spreads right after its own
-// interpolation, in the same warp.  Each CTA writes its sphere force/torque
-// partial to fpart[sphere][split][6]; k_ibm_update adds the partials in a fixed
-// order.
-__global__ void __launch_bounds__(IBM_THREADS) k_ibm_interp_spread(IbmParams P, const DPart* parts, const double* X,
-                                                                    const double* Y, const double* Z, const double* S,
-                                                                    double* nfx, double* nfy, double* nfz, double* ndx,
-                                                                    double* ndy, double* ndz, const float* fields,
-                                                                    unsigned long long* faux, double* fpart,
-                                                                    int split) {
+// The Lagrangian nodes' arrays.
+struct IbmNodes {
+    double *x, *y, *z;
+    const double* S;
+    double *fx, *fy, *fz;      // force of the step
+    double *dx, *dy, *dz;      // force of the last iteration
+};
+
+// Interpolation, direct forcing and spreading (ibm.cu:307-541) of one
+// Lagrangian node by a group of 16 lanes (lane l of the group); every lane of
+// the warp calls it (`active`: the group has a node).
+//
+// What bounds it is the chain of a node's dependent steps (position, stencil,
+// fields, sum, force, spread) and the instructions around it, so two nodes
+// share a warp and nothing is computed twice: lane l evaluates one of the 12
+// stencil factors and coordinates (axis l / 4, point l % 4) and the lanes
+// exchange them; lane l takes the points (x, y) = (l % 4, l / 4) of the four z
+// planes, so four neighbouring lanes read 64 contiguous bytes of the field
+// records and add to 32 contiguous bytes of each spread component; the four
+// sums are reduced by halves, after which lanes 4-15 hold u and evaluate one
+// component of the force each.  The interpolation reads the IBM macroscopic
+// records and the spreading adds into the auxiliary force field, two different
+// arrays, so each node spreads right after its own interpolation.  64 spheres
+// of radius 8 (38,912 nodes, three iterations) in 192x192x384: with one warp
+// per node, every lane evaluating all 12 factors, and fields as four planes, a
+// step took 0.94 ms; with this, the float4 records and a box node per thread in
+// the Eulerian pass 0.78 ms (31 us per launch of this kernel).
+// Returns in accF / accM the component (l / 4) - 1 of the node's force and
+// torque, added to what they hold (lanes 0-3: unused).
+__device__ __forceinline__ void interp_spread_node(const IbmParams& P, const DPart& p, const IbmNodes& nd, int j,
+                                                   bool active, int l, const float4* __restrict__ fields,
+                                                   unsigned long long* faux, double& accF, double& accM) {
+    constexpr unsigned ALL = 0xffffffffu;
+    const int half = threadIdx.x & 16;
+    const double pos3[3] = {nd.x[j], nd.y[j], nd.z[j]};
+    // this lane's axis and stencil point (lanes 12-15 repeat the z axis)
+    const int ax = min(l >> 2, 2), pt = l & 3;
+    float w;
+    int coord;      // lattice coordinate of the point, -1 outside a wall
+    bool skip = !active;
+    {
+        const double q = ax == 0 ? pos3[0] : (ax == 1 ? pos3[1] : pos3[2]);
+        const bool wall = ax == 0 ? P.wall[0] : (ax == 1 ? P.wall[1] : P.wall[2]);
+        const int Li = ax == 0 ? P.nx : (ax == 1 ? P.ny : P.nz);
+        const double L = (double)Li;
+        const double centre = p.pos[ax];
+        const double xu = wall ? q : centre + pdelta(q - centre, L);
+        const bool lost = !(fabs(xu) < 4.0 * L + 8.0);   // non-finite or diverged position: no stencil
+        // int(x) - P_DIST + 1 of the stored coordinate (ibm.cu:236-240): truncation,
+        // which differs from floor for the negative coordinates a sphere's nodes
+        // have across x=0 before their first movement wraps them; for periodic
+        // axes the base is then shifted into the sphere-centred frame
+        const double raw = lost ? 0.0 : q;
+        const int braw = (int)raw - 1;
+        int base = braw, lo = 0, hi = 3;
+        if (wall) {
+            hi = (base + 3 < Li) ? 3 : (Li - 1 - base);
+            lo = (base >= 0) ? 0 : -base;
+        } else if (!lost) {   // pdelta moved the coordinate by a period or not at all
+            const double d = xu - raw;
+            base += d > 0.5 * L ? Li : (d < -0.5 * L ? -Li : 0);
+        }
+        skip = skip || lost || hi <= 0 || lo >= 4;   // ibm.cu:300-305
+        w = stencil4((float)pt - (float)(raw - (double)braw));
+        coord = (pt >= lo && pt <= hi) ? wrap_near(base + pt, Li) : -1;
+    }
+    skip = ((__ballot_sync(ALL, skip) >> half) & 0xfffu) != 0;
+    const float wx = __shfl_sync(ALL, w, l & 3, IBM_NODE_LANES), wy = __shfl_sync(ALL, w, 4 + (l >> 2), IBM_NODE_LANES);
+    const int cx = __shfl_sync(ALL, coord, l & 3, IBM_NODE_LANES), cy = __shfl_sync(ALL, coord, 4 + (l >> 2), IBM_NODE_LANES);
+    const bool in_xy = !skip && cx >= 0 && cy >= 0;
+    unsigned g[4];
+    float d[4];
+    bool in[4];
+    float4 v[4];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        const float wz = __shfl_sync(ALL, w, 8 + h, IBM_NODE_LANES);
+        const int cz = __shfl_sync(ALL, coord, 8 + h, IBM_NODE_LANES);
+        in[h] = in_xy && cz >= 0;
+        d[h] = (wz * wy) * wx;
+        g[h] = in[h] ? (unsigned)((cz * P.ny + cy) * P.nx + cx) : 0u;   // the lattice has < 2^31 nodes
+        v[h] = in[h] ? fields[g[h]] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;   // rho, ux, uy, uz
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+        if (in[h]) {
+            s0 += v[h].x * d[h]; s1 += v[h].y * d[h];
+            s2 += v[h].z * d[h]; s3 += v[h].w * d[h];
+        }
+    // sums over the 16 lanes by halves: lanes 0-3 end with rho, 4-7 ux, 8-11 uy, 12-15 uz
+    const bool up8 = l & 8, up4 = l & 4;
+    float a = up8 ? s2 : s0, b = up8 ? s3 : s1;
+    a += __shfl_xor_sync(ALL, up8 ? s0 : s2, 8);
+    b += __shfl_xor_sync(ALL, up8 ? s1 : s3, 8);
+    float r = up4 ? b : a;
+    r += __shfl_xor_sync(ALL, up4 ? a : b, 4);
+    r += __shfl_xor_sync(ALL, r, 2);
+    r += __shfl_xor_sync(ALL, r, 1);
+    const float rho = __shfl_sync(ALL, r, 0, IBM_NODE_LANES);
+    // one component of the force per lane: c = (l / 4) - 1, with the cyclic neighbours c1, c2
+    const int c = max(l >> 2, 1) - 1, c1 = c == 2 ? 0 : c + 1, c2 = c == 0 ? 2 : c - 1;
+    double dr[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        dr[k] = pos3[k] - p.pos[k];
+        if (!P.wall[k]) dr[k] = pdelta(dr[k], (double)(k == 0 ? P.nx : (k == 1 ? P.ny : P.nz)));
+    }
+    const double dr1 = c == 0 ? dr[1] : (c == 1 ? dr[2] : dr[0]), dr2 = c == 0 ? dr[2] : (c == 1 ? dr[0] : dr[1]);
+    const double uc = p.movable ? p.vel[c] + (p.w[c1] * dr2 - p.w[c2] * dr1) : 0.0;
+    const double aux = 2.0 * (double)rho * nd.S[j] * P.thickness;
+    const double dF = aux * ((double)r - uc);
+    const double F[3] = {__shfl_sync(ALL, dF, 4, IBM_NODE_LANES), __shfl_sync(ALL, dF, 8, IBM_NODE_LANES),
+                         __shfl_sync(ALL, dF, 12, IBM_NODE_LANES)};
+    if (active && l >= 4 && (l & 3) == 0) {
+        double* out = c == 0 ? nd.dx : (c == 1 ? nd.dy : nd.dz);
+        out[j] = skip ? 0.0 : dF;
+        if (!skip) {
+            double* sum = c == 0 ? nd.fx : (c == 1 ? nd.fy : nd.fz);
+            sum[j] += dF;
+        }
+    }
+    if (skip) return;
+    const double F1 = c == 0 ? F[1] : (c == 1 ? F[2] : F[0]), F2 = c == 0 ? F[2] : (c == 1 ? F[0] : F[1]);
+    accF += dF;
+    accM += dr1 * F2 - dr2 * F1;
+    // spreading: fAux -= dF * delta (ibm.cu:478-512), in fixed point so the
+    // sum is the same in any order
+    const float f0 = (float)F[0], f1 = (float)F[1], f2 = (float)F[2];
+    const size_t N = (size_t)P.nx * P.ny * P.nz;
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+        if (in[h]) {
+            atomicAdd(&faux[g[h]], to_fix(-f0 * d[h]));
+            atomicAdd(&faux[N + g[h]], to_fix(-f1 * d[h]));
+            atomicAdd(&faux[2 * N + g[h]], to_fix(-f2 * d[h]));
+        }
+}
+
+// One forcing iteration over the Lagrangian nodes: `split` CTAs per sphere, a
+// group of lanes per node.  Each CTA writes its sphere force/torque partial to
+// fpart[sphere][split][6]; k_ibm_update adds the partials in a fixed order.
+__global__ void __launch_bounds__(IBM_THREADS) k_ibm_interp_spread(IbmParams P, const DPart* parts, IbmNodes nd,
+                                                                    const float4* fields, unsigned long long* faux,
+                                                                    double* fpart, int split) {
     chain_enter();
-    __shared__ double red[32];
+    constexpr int GROUPS = IBM_THREADS / IBM_NODE_LANES;
+    __shared__ double red[GROUPS][6];
     const int sphere = blockIdx.x / split, sub = blockIdx.x % split;
     const DPart& p = parts[sphere];
-    const size_t N = (size_t)P.nx * P.ny * P.nz;
-    const float* rho_g = fields;
-    const float* ux_g = fields + N;
-    const float* uy_g = fields + 2 * N;
-    const float* uz_g = fields + 3 * N;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int warps = IBM_THREADS / 32;
-    const double L[3] = {(double)P.nx, (double)P.ny, (double)P.nz};
-    double accF[3] = {0, 0, 0}, accM[3] = {0, 0, 0};
+    const int l = threadIdx.x & (IBM_NODE_LANES - 1), group = threadIdx.x / IBM_NODE_LANES;
+    double accF = 0.0, accM = 0.0;
     const int nb = p.node_count;
-    for (int k = sub * warps + warp; k < nb; k += split * warps) {
-        const int j = p.node_begin + k;
-        const double xj = X[j], yj = Y[j], zj = Z[j];
-        const NodeStencil st = node_stencil(P, p, xj, yj, zj);
-        if (st.skip) {
-            if (lane == 0) ndx[j] = ndy[j] = ndz[j] = 0.0;
-            continue;
-        }
-        size_t g[2];
-        float d[2];
-        bool in[2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int q = lane + 32 * h;
-            const int xi = q & 3, yi = (q >> 2) & 3, zi = q >> 4;
-            in[h] = xi >= st.lo[0] && xi <= st.hi[0] && yi >= st.lo[1] && yi <= st.hi[1] && zi >= st.lo[2] &&
-                    zi <= st.hi[2];
-            d[h] = (st.w[2][zi] * st.w[1][yi]) * st.w[0][xi];
-            const int x = wrap_near(st.base[0] + xi, P.nx), y = wrap_near(st.base[1] + yi, P.ny),
-                      z = wrap_near(st.base[2] + zi, P.nz);
-            g[h] = ((size_t)z * P.ny + y) * P.nx + x;
-        }
-        float rho = 0.f, ux = 0.f, uy = 0.f, uz = 0.f;
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-            if (in[h]) {
-                rho += rho_g[g[h]] * d[h]; ux += ux_g[g[h]] * d[h];
-                uy += uy_g[g[h]] * d[h]; uz += uz_g[g[h]] * d[h];
-            }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            rho += __shfl_xor_sync(0xffffffffu, rho, o);
-            ux += __shfl_xor_sync(0xffffffffu, ux, o);
-            uy += __shfl_xor_sync(0xffffffffu, uy, o);
-            uz += __shfl_xor_sync(0xffffffffu, uz, o);
-        }
-        double dr[3] = {xj - p.pos[0], yj - p.pos[1], zj - p.pos[2]};
-        for (int a = 0; a < 3; ++a)
-            if (!P.wall[a]) dr[a] = pdelta(dr[a], L[a]);
-        double uc[3] = {0, 0, 0};
-        if (p.movable) {
-            double wxr[3];
-            dcross(p.w, dr, wxr);
-            for (int a = 0; a < 3; ++a) uc[a] = p.vel[a] + wxr[a];
-        }
-        const double aux = 2.0 * (double)rho * S[j] * P.thickness;
-        const double dF[3] = {aux * ((double)ux - uc[0]), aux * ((double)uy - uc[1]), aux * ((double)uz - uc[2])};
-        if (lane == 0) {
-            nfx[j] += dF[0]; nfy[j] += dF[1]; nfz[j] += dF[2];
-            ndx[j] = dF[0]; ndy[j] = dF[1]; ndz[j] = dF[2];
-            double m[3];
-            dcross(dr, dF, m);
-            for (int a = 0; a < 3; ++a) { accF[a] += dF[a]; accM[a] += m[a]; }
-        }
-        // spreading: fAux -= dF * delta (ibm.cu:478-512), in fixed point so the
-        // sum is the same in any order
-        const float f0 = (float)dF[0], f1 = (float)dF[1], f2 = (float)dF[2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-            if (in[h]) {
-                atomicAdd(&faux[g[h]], to_fix(-f0 * d[h]));
-                atomicAdd(&faux[N + g[h]], to_fix(-f1 * d[h]));
-                atomicAdd(&faux[2 * N + g[h]], to_fix(-f2 * d[h]));
-            }
+    for (int k0 = sub * GROUPS + (group & ~1); k0 < nb; k0 += split * GROUPS) {   // both groups of a warp together
+        const int k = k0 + (group & 1);
+        interp_spread_node(P, p, nd, p.node_begin + min(k, nb - 1), k < nb, l, fields, faux, accF, accM);
     }
-    // this CTA's part of the sphere force and torque (ibm.cu:526-541)
-    double tot6[6];
-    for (int a = 0; a < 3; ++a) { tot6[a] = block_sum(accF[a], red); tot6[3 + a] = block_sum(accM[a], red); }
-    if (threadIdx.x == 0)
-        for (int a = 0; a < 6; ++a) fpart[((size_t)sphere * split + sub) * 6 + a] = tot6[a];
+    if (l >= 4 && (l & 3) == 0) {
+        red[group][(l >> 2) - 1] = accF;
+        red[group][(l >> 2) + 2] = accM;
+    }
+    __syncthreads();
+    if (threadIdx.x < 6) {   // this CTA's part of the sphere force and torque (ibm.cu:526-541)
+        double t = 0.0;
+        for (int k = 0; k < GROUPS; ++k) t += red[k][threadIdx.x];
+        fpart[((size_t)sphere * split + sub) * 6 + threadIdx.x] = t;
+    }
 }
 
 // gpuParticleMovement ibm.cu:899-993
@@ -818,7 +843,28 @@ __device__ void move_node(const IbmParams& P, const DPart* parts, const int* pid
 // After the last forcing iteration the same launch moves the Lagrangian nodes
 // (gpuParticleNodeMovement ibm.cu:1044-1197), which k_ibm_update's particle
 // movement precedes, and releases the owners.  `split` CTAs per sphere.
-__global__ void __launch_bounds__(IBM_THREADS) k_ibm_euler(IbmParams P, float* fields, unsigned long long* faux,
+__device__ __forceinline__ void euler_node(size_t N, unsigned n, unsigned sphere, float4* fields,
+                                           unsigned long long* faux, float* fibm, uint8_t* cls, unsigned* owner,
+                                           int last) {
+    // loaded together: one trip to memory before the branch, not two
+    const unsigned own = owner[n];
+    const unsigned long long a0 = faux[n], a1 = faux[N + n], a2 = faux[2 * N + n];
+    if (own != sphere) return;
+    if (last) owner[n] = IBM_NO_OWNER;
+    if ((a0 | a1 | a2) == 0ull) return;
+    float4 m = fields[n];
+    const float v0 = from_fix(a0), v1 = from_fix(a1), v2 = from_fix(a2);
+    m.y += 0.5f * v0 / m.x;
+    m.z += 0.5f * v1 / m.x;
+    m.w += 0.5f * v2 / m.x;
+    fields[n] = m;
+    fibm[n] += v0;
+    fibm[N + n] += v1;
+    fibm[2 * N + n] += v2;
+    faux[n] = faux[N + n] = faux[2 * N + n] = 0ull;
+    cls[n] = cls[n] | NODE_IBM_FORCE;
+}
+__global__ void __launch_bounds__(IBM_THREADS) k_ibm_euler(IbmParams P, float4* fields, unsigned long long* faux,
                                                             float* fibm, uint8_t* cls, unsigned* owner,
                                                             const DPart* parts, const int* pid, double* X, double* Y,
                                                             double* Z, int split, int last) {
@@ -829,41 +875,43 @@ __global__ void __launch_bounds__(IBM_THREADS) k_ibm_euler(IbmParams P, float* f
             move_node(P, parts, pid, X, Y, Z, k);
     const unsigned sphere = blockIdx.x / split;
     const DPart& p = parts[sphere];
-    const int sub = blockIdx.x % split;
     const unsigned tot = box_size(p);
-    for (unsigned k = sub * blockDim.x + threadIdx.x; k < tot; k += split * blockDim.x) {
-        const unsigned n = box_node(P, p, k);
-        if (owner[n] != sphere) continue;
-        if (last) owner[n] = IBM_NO_OWNER;
-        const unsigned long long a0 = faux[n], a1 = faux[N + n], a2 = faux[2 * N + n];
-        if ((a0 | a1 | a2) == 0ull) continue;
-        const float rho = fields[n];
-        const unsigned long long av[3] = {a0, a1, a2};
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            const float v = from_fix(av[a]);
-            fields[(1 + a) * N + n] += 0.5f * v / rho;
-            fibm[a * N + n] += v;
-            faux[a * N + n] = 0ull;
-        }
-        cls[n] = cls[n] | NODE_IBM_FORCE;
-    }
+    for (unsigned k = (blockIdx.x % split) * blockDim.x + threadIdx.x; k < tot; k += split * blockDim.x)
+        euler_node(N, box_node(P, p, k), sphere, fields, faux, fibm, cls, owner, last);
 }
 
 // The IBM macroscopics of this step's box nodes into the caller's arrays.
-__global__ void __launch_bounds__(IBM_THREADS) k_ibm_fixup(IbmParams P, const DPart* parts, const float* fields,
+__global__ void __launch_bounds__(IBM_THREADS) k_ibm_fixup(IbmParams P, const DPart* parts, const float4* fields,
                                                             int split, float* rho, float* ux, float* uy, float* uz) {
-    const size_t N = (size_t)P.nx * P.ny * P.nz;
     const DPart& p = parts[blockIdx.x / split];
     const int sub = blockIdx.x % split;
     const unsigned tot = box_size(p);
     for (unsigned k = sub * blockDim.x + threadIdx.x; k < tot; k += split * blockDim.x) {
         const unsigned n = box_node(P, p, k);
-        if (rho) rho[n] = fields[n];
-        if (ux) ux[n] = fields[N + n];
-        if (uy) uy[n] = fields[2 * N + n];
-        if (uz) uz[n] = fields[3 * N + n];
+        const float4 m = fields[n];
+        if (rho) rho[n] = m.x;
+        if (ux) ux[n] = m.y;
+        if (uy) uy[n] = m.z;
+        if (uz) uz[n] = m.w;
     }
+}
+
+// The IBM macroscopics as planes [4][N] (a checkpoint image keeps them so) from
+// the records, or back.
+__global__ void __launch_bounds__(IBM_THREADS) k_ibm_planes(float4* fields, float* planes, size_t N, int to_planes) {
+    const size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= N) return;
+    if (to_planes) {
+        const float4 m = fields[n];
+        planes[n] = m.x; planes[N + n] = m.y; planes[2 * N + n] = m.z; planes[3 * N + n] = m.w;
+    } else {
+        fields[n] = make_float4(planes[n], planes[N + n], planes[2 * N + n], planes[3 * N + n]);
+    }
+}
+cudaError_t ibm_planes(void* fields, float* planes, size_t N, bool to_planes, cudaStream_t s) {
+    k_ibm_planes<<<(unsigned)((N + IBM_THREADS - 1) / IBM_THREADS), IBM_THREADS, 0, s>>>(
+        static_cast<float4*>(fields), planes, N, to_planes ? 1 : 0);
+    return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------- host --
@@ -953,6 +1001,10 @@ static cudaError_t gather_dispatch(vlbm_sim* s, IbmState* st) {
     return launch_gather<27, VLBM_STORE_BF16>(s, st);
 }
 
+static IbmNodes ibm_nodes(const IbmState* st) {
+    return IbmNodes{st->nx, st->ny, st->nz, st->nS, st->nfx, st->nfy, st->nfz, st->ndx, st->ndy, st->ndz};
+}
+
 vlbm_status ibm_step(vlbm_sim* s) {
     IbmState* st = s->ibm;
     if (!st || st->np == 0) return VLBM_OK;
@@ -975,9 +1027,7 @@ vlbm_status ibm_step(vlbm_sim* s) {
     for (int it = 0; it < iters; ++it) {
         const int last = it == iters - 1;
         IBM_CUDA(launch_chained(k_ibm_interp_spread, st->np * st->split, cs, P, (const DPart*)st->parts,
-                                (const double*)st->nx, (const double*)st->ny, (const double*)st->nz,
-                                (const double*)st->nS, st->nfx, st->nfy, st->nfz, st->ndx, st->ndy, st->ndz,
-                                (const float*)st->fields, st->faux, st->fpart, st->split));
+                                ibm_nodes(st), (const float4*)st->fields, st->faux, st->fpart, st->split));
         IBM_CUDA(launch_chained(k_ibm_update, (st->np + IBM_THREADS / 32 - 1) / (IBM_THREADS / 32), cs, P, st->parts,
                                 (const double*)st->fpart, st->split, last, st->clock));
         IBM_CUDA(launch_chained(k_ibm_euler, st->np * st->gsplit, cs, P, st->fields, st->faux, s->fibm, s->cls,
@@ -1046,7 +1096,7 @@ void ibm_state_regions(vlbm_sim* s, std::vector<StateRegion>& out) {
     for (double* p : {st->nx, st->ny, st->nz, st->nS, st->nfx, st->nfy, st->nfz, st->ndx, st->ndy, st->ndz})
         out.push_back({id++, p, nn * sizeof(double)});
     out.push_back({111, st->npid, nn * sizeof(int)});
-    out.push_back({112, st->fields, 4 * N * sizeof(float)});
+    out.push_back({112, st->fields, 4 * N * sizeof(float), true});
     out.push_back({114, st->clock, sizeof(int)});
 }
 
@@ -1085,7 +1135,7 @@ void ibm_reset(vlbm_sim* s) {
     cudaMemcpyAsync(st->nx, st->init_nodes.data(), nn * sizeof(double), cudaMemcpyHostToDevice, s->stream);
     cudaMemcpyAsync(st->ny, st->init_nodes.data() + nn, nn * sizeof(double), cudaMemcpyHostToDevice, s->stream);
     cudaMemcpyAsync(st->nz, st->init_nodes.data() + 2 * nn, nn * sizeof(double), cudaMemcpyHostToDevice, s->stream);
-    cudaMemsetAsync(st->fields, 0, (size_t)4 * s->N * sizeof(float), s->stream);
+    cudaMemsetAsync(st->fields, 0, (size_t)s->N * sizeof(float4), s->stream);
     cudaMemsetAsync(st->faux, 0, (size_t)3 * s->N * sizeof(unsigned long long), s->stream);
     cudaMemsetAsync(st->owner, 0xFF, (size_t)s->N * sizeof(unsigned), s->stream);   // IBM_NO_OWNER
     cudaMemsetAsync(st->clock, 0, sizeof(int), s->stream);
@@ -1201,7 +1251,7 @@ vlbm_status vlbm_add_spheres(vlbm_sim* s, const vlbm_ibm_config* ib, const vlbm_
     for (double** d : dp)
         if (e == cudaSuccess) e = dalloc((void**)d, nn * sizeof(double));
     if (e == cudaSuccess) e = dalloc((void**)&st->npid, nn * sizeof(int));
-    if (e == cudaSuccess) e = dalloc((void**)&st->fields, 4 * N * sizeof(float));
+    if (e == cudaSuccess) e = dalloc((void**)&st->fields, N * sizeof(float4));
     if (e == cudaSuccess) e = dalloc((void**)&st->faux, 3 * N * sizeof(unsigned long long));
     if (e == cudaSuccess) e = dalloc((void**)&st->owner, N * sizeof(unsigned));
     if (e == cudaSuccess) e = dalloc((void**)&st->clock, sizeof(int));
@@ -1218,14 +1268,14 @@ vlbm_status vlbm_add_spheres(vlbm_sim* s, const vlbm_ibm_config* ib, const vlbm_
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&st->cstream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&st->ev_fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&st->ev_join, cudaEventDisableTiming);
-    {   // CTAs per sphere of the box passes: about two box nodes per thread for the largest sphere
+    {   // CTAs per sphere of the box passes: about one box node per thread for the largest sphere
         long long maxbox = 1;
         for (int k = 0; k < n; ++k) {
             const long long side = (long long)std::ceil(sp[k].diameter) + 6;
             maxbox = std::max(maxbox, std::min<long long>(side, c.nx) * std::min<long long>(side, c.ny) *
                                           std::min<long long>(side, c.nz));
         }
-        st->gsplit = (int)std::min<long long>(IBM_MAX_SPLIT, std::max<long long>(1, maxbox / (2 * IBM_THREADS)));
+        st->gsplit = (int)std::min<long long>(IBM_MAX_SPLIT, std::max<long long>(1, (maxbox + IBM_THREADS - 1) / IBM_THREADS));
     }
     if (e == cudaSuccess && !s->fibm) {
         e = sim_malloc(s, (void**)&s->fibm, 3 * N * sizeof(float));
@@ -1243,7 +1293,7 @@ vlbm_status vlbm_add_spheres(vlbm_sim* s, const vlbm_ibm_config* ib, const vlbm_
     if (e == cudaSuccess) e = sim_upload(s, st->nz, Z.data(), nn * sizeof(double));
     if (e == cudaSuccess) e = sim_upload(s, st->nS, S.data(), nn * sizeof(double));
     if (e == cudaSuccess) e = sim_upload(s, st->npid, pid.data(), nn * sizeof(int));
-    if (e == cudaSuccess) e = cudaMemsetAsync(st->fields, 0, 4 * N * sizeof(float), ss);
+    if (e == cudaSuccess) e = cudaMemsetAsync(st->fields, 0, N * sizeof(float4), ss);
     if (e == cudaSuccess) e = cudaMemsetAsync(st->faux, 0, 3 * N * sizeof(unsigned long long), ss);
     if (e == cudaSuccess) e = cudaMemsetAsync(st->owner, 0xFF, N * sizeof(unsigned), ss);   // IBM_NO_OWNER
     if (e == cudaSuccess) e = sim_upload(s, st->clock, &clock, sizeof(int));

@@ -124,11 +124,14 @@ struct StateRegion {
     uint32_t id;
     void* dev;
     size_t bytes;
+    bool records4 = false;   // float4 per node on the device, four planes in the image
 };
 
 // IBM hooks (ibm.cu)
 void ibm_state_regions(vlbm_sim* s, std::vector<StateRegion>& out);
 uint32_t ibm_record_bytes();   // bytes of one device particle record
+// float4 records of N nodes to planes [4][N] or back (device pointers).
+cudaError_t ibm_planes(void* fields, float* planes, size_t N, bool to_planes, cudaStream_t s);
 vlbm_status ibm_step(vlbm_sim* s);
 vlbm_status ibm_macroscopics_fixup(vlbm_sim* s, float* rho, float* ux, float* uy, float* uz);
 void ibm_destroy(IbmState* st, DeviceAllocator* allocator);
