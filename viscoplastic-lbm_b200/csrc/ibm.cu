@@ -244,7 +244,7 @@ __device__ __forceinline__ void gather_box_node(const StepParams& sp, const IbmP
     nb.init(x, y, z, sp.nx, sp.ny, sp.nz);
     float f[Q];
     uint8_t cls;
-    gather<Q, ST, ODD, PAIRED>(sp, n, nb, x, y, z, f, cls);
+    gather_node<Q, ST, ODD, PAIRED>(sp, n, nb, x, y, z, f, cls);
     const Mom m = moments<Q, false>(f, P.fx, P.fy, P.fz, sp.rho0);
     fields[n] = make_float4(m.rho, m.ux, m.uy, m.uz);
     atomicMin(&owner[n], sphere);
@@ -625,7 +625,7 @@ struct IbmNodes {
 // Returns in accF / accM the component (l / 4) - 1 of the node's force and
 // torque, added to what they hold (lanes 0-3: unused).
 __device__ __forceinline__ void interp_spread_node(const IbmParams& P, const DPart& p, const IbmNodes& nd, int j,
-                                                   bool active, int l, const float4* __restrict__ fields,
+                                                   bool active, int l, const float4* fields,
                                                    unsigned long long* faux, double& accF, double& accM) {
     constexpr unsigned ALL = 0xffffffffu;
     const int half = threadIdx.x & 16;
@@ -975,34 +975,33 @@ static cudaError_t launch_chained(void (*kernel)(KArgs...), unsigned grid, cudaS
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-template <int Q, int ST>
+static IbmNodes ibm_nodes(const IbmState* st) {
+    return IbmNodes{st->nx, st->ny, st->nz, st->nS, st->nfx, st->nfy, st->nfz, st->ndx, st->ndy, st->ndz};
+}
+
+template <int Q, int ST, bool ODD, bool PAIRED>
 static cudaError_t launch_gather(vlbm_sim* s, IbmState* st) {
-    const StepParams sp = make_params(s);
-    const bool pr = sp.pairH > 0;
-    if (s->parity == 1) {
-        if (pr) return launch_chained(k_ibm_gather<Q, ST, true, true>, st->np * st->gsplit, s->stream, sp, st->prm, (const DPart*)st->parts, st->fields, st->owner, st->gsplit);
-        else return launch_chained(k_ibm_gather<Q, ST, true, false>, st->np * st->gsplit, s->stream, sp, st->prm, (const DPart*)st->parts, st->fields, st->owner, st->gsplit);
-    } else {
-        if (pr) return launch_chained(k_ibm_gather<Q, ST, false, true>, st->np * st->gsplit, s->stream, sp, st->prm, (const DPart*)st->parts, st->fields, st->owner, st->gsplit);
-        else return launch_chained(k_ibm_gather<Q, ST, false, false>, st->np * st->gsplit, s->stream, sp, st->prm, (const DPart*)st->parts, st->fields, st->owner, st->gsplit);
-    }
-    return cudaGetLastError();
+    return launch_chained(k_ibm_gather<Q, ST, ODD, PAIRED>, st->np * st->gsplit, s->stream, make_params(s), st->prm,
+                          (const DPart*)st->parts, st->fields, st->owner, st->gsplit);
+}
+
+template <int Q, int ST>
+static cudaError_t gather_family(vlbm_sim* s, IbmState* st) {
+    const bool pr = s->pairH > 0;
+    if (s->parity == 1) return pr ? launch_gather<Q, ST, true, true>(s, st) : launch_gather<Q, ST, true, false>(s, st);
+    return pr ? launch_gather<Q, ST, false, true>(s, st) : launch_gather<Q, ST, false, false>(s, st);
 }
 
 static cudaError_t gather_dispatch(vlbm_sim* s, IbmState* st) {
     const int sto = s->cfg.storage;
     if (s->Q == 19) {
-        if (sto == VLBM_STORE_F32) return launch_gather<19, VLBM_STORE_F32>(s, st);
-        if (sto == VLBM_STORE_F16) return launch_gather<19, VLBM_STORE_F16>(s, st);
-        return launch_gather<19, VLBM_STORE_BF16>(s, st);
+        if (sto == VLBM_STORE_F32) return gather_family<19, VLBM_STORE_F32>(s, st);
+        if (sto == VLBM_STORE_F16) return gather_family<19, VLBM_STORE_F16>(s, st);
+        return gather_family<19, VLBM_STORE_BF16>(s, st);
     }
-    if (sto == VLBM_STORE_F32) return launch_gather<27, VLBM_STORE_F32>(s, st);
-    if (sto == VLBM_STORE_F16) return launch_gather<27, VLBM_STORE_F16>(s, st);
-    return launch_gather<27, VLBM_STORE_BF16>(s, st);
-}
-
-static IbmNodes ibm_nodes(const IbmState* st) {
-    return IbmNodes{st->nx, st->ny, st->nz, st->nS, st->nfx, st->nfy, st->nfz, st->ndx, st->ndy, st->ndz};
+    if (sto == VLBM_STORE_F32) return gather_family<27, VLBM_STORE_F32>(s, st);
+    if (sto == VLBM_STORE_F16) return gather_family<27, VLBM_STORE_F16>(s, st);
+    return gather_family<27, VLBM_STORE_BF16>(s, st);
 }
 
 vlbm_status ibm_step(vlbm_sim* s) {

@@ -453,36 +453,15 @@ __global__ void __launch_bounds__(256) k_halo(void* pop, HaloMsg m0, HaloMsg m1,
     if (unpack) P[e] = B[t];
     else B[t] = P[e];
 }
-__device__ __forceinline__ int wrap1(int v, int n) { return v < 0 ? v + n : (v >= n ? v - n : v); }
 
-// Gather f_i(x, t) of node n (after boundary rules).  Returns the side-store
+// Gather f_i(x, t) of node n of a natural-layout state (after boundary rules).  Returns the side-store
 // slot of a boundary node, -1 for bulk nodes.
-template <int Q, int ST, bool ODD, bool PAIRED = false>
+template <int Q, int ST, bool ODD>
 __device__ __forceinline__ int gather(const StepParams& p, const float* side_prev, int use_bc, unsigned n,
                                       const Nbr& nb, int x, int y, int z, float (&f)[Q], uint8_t& cls) {
     using S = Store<ST>;
     using T = typename S::T;
     const size_t N = (size_t)p.N;
-    if (PAIRED) {
-        const T* A = static_cast<const T*>(p.pop);
-#pragma unroll
-        for (int i = 0; i < Q; ++i) {
-            if (!ODD) {
-                f[i] = S::ld(A + pair_elem<Q>(p, i, x, y, z), Lattice<Q>::w(i), p);
-            } else {
-                const size_t src = pair_elem<Q>(p, lat_opp(i), wrap1(x - lat_cx(i), p.nx), wrap1(y - lat_cy(i), p.ny),
-                                                wrap1(z - lat_cz(i), p.nz));
-                f[i] = S::ld(A + src, Lattice<Q>::w(i), p);
-            }
-        }
-        cls = p.cls[n];
-        int slot = -1;
-        if (cls & NODE_BC) {
-            slot = p.bc_slot[n];
-            if (use_bc) apply_bc<Q>(f, p, side_prev, slot, x, y, z, nb, n);
-        }
-        return slot;
-    }
     // walk the planes with one running pointer: plane j holds population j in
     // the natural layout (even steps) and population opp(j) after an even step
     const T* plane = static_cast<const T*>(p.pop);
@@ -504,10 +483,10 @@ __device__ __forceinline__ int gather(const StepParams& p, const float* side_pre
     }
     return slot;
 }
-template <int Q, int ST, bool ODD, bool PAIRED = false>
+template <int Q, int ST, bool ODD>
 __device__ __forceinline__ int gather(const StepParams& p, unsigned n, const Nbr& nb, int x, int y, int z,
                                       float (&f)[Q], uint8_t& cls) {
-    return gather<Q, ST, ODD, PAIRED>(p, p.side_prev, p.apply_bc, n, nb, x, y, z, f, cls);
+    return gather<Q, ST, ODD>(p, p.side_prev, p.apply_bc, n, nb, x, y, z, f, cls);
 }
 
 // Moments of a node: rho, u (with half force, lbm.cu:79-111), non-equilibrium
@@ -1069,11 +1048,14 @@ struct PairNode {
     Nbr pn;                       // neighbour offsets in pair space
     BlkNbr bn;
     __device__ __forceinline__ void init(const StepParams& p, unsigned m_) {
+        const unsigned t = m_ / (unsigned)p.nx;
+        init_at(p, m_, (int)(m_ % (unsigned)p.nx), (int)(t % (unsigned)p.ny), (int)(t / (unsigned)p.ny));
+    }
+    __device__ __forceinline__ void init_at(const StepParams& p, unsigned m_, int x_, int y_, int zp_) {
         m = m_;
-        x = (int)(m % (unsigned)p.nx);
-        const unsigned t = m / (unsigned)p.nx;
-        y = (int)(t % (unsigned)p.ny);
-        zp = (int)(t / (unsigned)p.ny);
+        x = x_;
+        y = y_;
+        zp = zp_;
         pn.init(x, y, zp, p.nx, p.ny, p.pairH);
         seam_lo = zp == 0;
         seam_hi = zp == p.pairH - 1;
@@ -1112,7 +1094,48 @@ struct PairNode {
             }
         }
     }
+    // The same for one node of the pair, as deviations.
+    __device__ __forceinline__ void load_lane(const StepParams& p, int lane, float (&f)[Q]) const {
+        using T = typename Store<ST>::T;
+        const T* A = static_cast<const T*>(p.pop);
+#pragma unroll
+        for (int j = 0; j < Q; ++j) {
+            const int i = ODD ? lat_opp(j) : j;
+            const int cx = lat_cx(i), cy = lat_cy(i), cz = lat_cz(i);
+            size_t e;   // pair
+            if (BLK) e = own + (ptrdiff_t)((ODD ? bn.off(-cx, -cy, -cz) : 0) + 32 * j);
+            else e = (size_t)j * Np + (unsigned)((int)m + (ODD ? pn.off(-cx, -cy, -cz) : 0));
+            const int other = ODD && ((cz > 0 && seam_lo) || (cz < 0 && seam_hi));
+            f[i] = Store<ST>::ld(A + 2 * e + (lane ^ other), Lattice<Q>::w(i), p);
+        }
+    }
 };
+
+// Gather f_i(x, t) of one node in any layout (after boundary rules): the
+// read-outs of scattered nodes and the reductions.
+template <int Q, int ST, bool ODD, bool PAIRED>
+__device__ __forceinline__ int gather_node(const StepParams& p, unsigned n, const Nbr& nb, int x, int y, int z,
+                                           float (&f)[Q], uint8_t& cls) {
+    if (!PAIRED) return gather<Q, ST, ODD>(p, n, nb, x, y, z, f, cls);
+    const int lane = z >= p.pairH ? 1 : 0, zp = z - lane * p.pairH;
+    const unsigned m = n - (lane ? (unsigned)(p.N >> 1) : 0u);
+    if (p.pairBlk) {
+        PairNode<Q, ST, ODD, true> pr;
+        pr.init_at(p, m, x, y, zp);
+        pr.load_lane(p, lane, f);
+    } else {
+        PairNode<Q, ST, ODD, false> pr;
+        pr.init_at(p, m, x, y, zp);
+        pr.load_lane(p, lane, f);
+    }
+    cls = p.cls[n];
+    int slot = -1;
+    if (cls & NODE_BC) {
+        slot = p.bc_slot[n];
+        if (p.apply_bc) apply_bc<Q>(f, p, slot, x, y, z, nb, n);
+    }
+    return slot;
+}
 
 // The boundary rules of a pair's boundary nodes, per lane on scalars, and their
 // side-store slots (-1: no boundary node).
