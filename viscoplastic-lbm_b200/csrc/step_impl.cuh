@@ -489,77 +489,6 @@ __device__ __forceinline__ int gather(const StepParams& p, unsigned n, const Nbr
     return gather<Q, ST, ODD>(p, p.side_prev, p.apply_bc, n, nb, x, y, z, f, cls);
 }
 
-// Moments of a node: rho, u (with half force, lbm.cu:79-111), non-equilibrium
-// second moments (lbm.cu:149-190) and the stress magnitude used by the
-// rheology models (lbm.cu:192-208).
-struct Mom {
-    float rho, drho, ux, uy, uz;
-    float pxx, pyy, pzz, pxy, pxz, pyz;
-};
-
-// Moments of the deviations g_i = f_i - w_i rho0: rho = rho0 + sum g,
-// rho u = sum c g + F/2, and the non-equilibrium second moments
-// Pi_ab = sum c_a c_b f - rho (u_a u_b + delta_ab / 3)
-//       = sum c_a c_b g - rho u_a u_b - delta_ab (rho - rho0) / 3.
-template <int Q, bool NEED_PI>
-__device__ __forceinline__ Mom moments(const float (&f)[Q], float fx, float fy, float fz, float rho0) {
-    // Sums over opposite pairs: e = g_i + g_opp feeds the even moments (rho,
-    // second moments), o = g_i - g_opp the odd ones (momentum).
-    Mom m;
-    float rho = f[0], jx = 0.f, jy = 0.f, jz = 0.f;
-    float sxx = 0.f, syy = 0.f, szz = 0.f, sxy = 0.f, sxz = 0.f, syz = 0.f;
-#pragma unroll
-    for (int i = 1; i < Q; i += 2) {
-        const int cx = lat_cx(i), cy = lat_cy(i), cz = lat_cz(i);
-        const float e = f[i] + f[i + 1], o = f[i] - f[i + 1];
-        rho += e;
-        if (cx) jx += cx * o;
-        if (cy) jy += cy * o;
-        if (cz) jz += cz * o;
-        if (NEED_PI) {
-            if (cx) sxx += e;
-            if (cy) syy += e;
-            if (cz) szz += e;
-            if (cx && cy) sxy += cx * cy * e;
-            if (cx && cz) sxz += cx * cz * e;
-            if (cy && cz) syz += cy * cz * e;
-        }
-    }
-    // correctly rounded reciprocal: u = j/rho enters every equilibrium, and a
-    // biased approximate reciprocal (the hardware MUFU result is within 2 ulp
-    // but not unbiased) acts like a spurious force proportional to the
-    // momentum, which shifts a slow channel flow by ~1e-3 over 1e4 steps
-    const float drho = rho;
-    rho += rho0;
-    const float inv = __frcp_rn(rho);
-    m.rho = rho;
-    m.drho = drho;
-    m.ux = (jx + 0.5f * fx) * inv;
-    m.uy = (jy + 0.5f * fy) * inv;
-    m.uz = (jz + 0.5f * fz) * inv;
-    if (NEED_PI) {
-        const float dr3 = drho * (1.f / 3.f);
-        m.pxx = sxx - rho * m.ux * m.ux - dr3;
-        m.pyy = syy - rho * m.uy * m.uy - dr3;
-        m.pzz = szz - rho * m.uz * m.uz - dr3;
-        m.pxy = sxy - rho * m.ux * m.uy;
-        m.pxz = sxz - rho * m.ux * m.uz;
-        m.pyz = syz - rho * m.uy * m.uz;
-    } else {
-        m.pxx = m.pyy = m.pzz = m.pxy = m.pxz = m.pyz = 0.f;
-    }
-    return m;
-}
-
-__device__ __forceinline__ float stress_aux(const Mom& m, float fx, float fy, float fz) {
-    const float a = m.pxx + m.ux * fx, b = m.pyy + m.uy * fy, c = m.pzz + m.uz * fz;
-    const float d = m.pxy + 0.5f * (m.ux * fy + m.uy * fx);
-    const float e = m.pxz + 0.5f * (m.ux * fz + m.uz * fx);
-    const float g = m.pyz + 0.5f * (m.uy * fz + m.uz * fy);
-    const float q = 0.5f * (a * a + b * b + c * c + 2.f * (d * d + e * e + g * g));
-    return q > 0.f ? q * rsqrtf(q) : 0.f;  // hardware reciprocal square root (<= 2 ulp)
-}
-
 // nnf.h:32-87 calcOmega.  For Power-Law the per-node state is the apparent
 // viscosity eta of the previous step (the reference stores omega,
 // lbm.cu:215-219); with omega_old = 1/(1/2 + 3 eta_old) the reference's
@@ -581,74 +510,6 @@ __device__ __forceinline__ float relax(const StepParams& p, float eta_old, float
         return 1.f / (0.5f + 3.f * eta_new);
     }
     return p.omega_newt;
-}
-
-// Collision in place: f <- f*.
-//  regularized (lbm.cu:263-461):
-//    f*_i = w_i [ A (Q_i:Pi - c_i.F/3) + rho(1 - 1.5u^2 + 3cu + 4.5cu^2) + B(3(c_i-u).F + 9 cu cF) ]
-//    A = 4.5(1-omega), B = 1-omega/2
-//  BGK (collisionForceNoReg.txt): f*_i = (1-omega) f_i + omega f_eq_i + B F_i
-template <int Q, int OP>
-__device__ __forceinline__ void collide(float (&f)[Q], const Mom& m, float omega, float fx, float fy, float fz) {
-    // Populations i (odd index) and opp(i) = i+1 have opposite velocities: they
-    // share Q_i:Pi, while c.u and c.F change sign.  Each pair is evaluated as an
-    // even part E and an odd part O with f*_i = w (E + O), f*_opp = w (E - O).
-    const float B = 1.f - 0.5f * omega;
-    const float uu = m.ux * m.ux + m.uy * m.uy + m.uz * m.uz;
-    const float uF = m.ux * fx + m.uy * fy + m.uz * fz;
-    if (OP == VLBM_OP_REGULARIZED) {
-        const float A = 4.5f * (1.f - omega);
-        const float tr = (m.pxx + m.pyy + m.pzz) * (1.f / 3.f);
-        // the rest part w_i rho0 is not formed: K0 is the deviation of rho(1 - 1.5 u^2)
-        const float K0 = m.drho - 1.5f * m.rho * uu - 3.f * B * uF - A * tr;
-        const float alpha = 3.f * B - A * (1.f / 3.f);
-        const float r3 = 3.f * m.rho, r45 = 4.5f * m.rho, b9 = 9.f * B;
-        f[0] = Lattice<Q>::w(0) * K0;
-        // coefficients with the weight of each velocity class folded in
-        float cK[3], cA[3], cr45[3], cb9[3], cal[3], cr3[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            // representative population of the class: 1 (axis), 7 (face), 19 (body, D3Q27 only)
-            const float w = Lattice<Q>::w(k == 0 ? 1 : (k == 1 ? 7 : (Q == 27 ? 19 : 1)));
-            cK[k] = w * K0; cA[k] = w * A; cr45[k] = w * r45; cb9[k] = w * b9; cal[k] = w * alpha; cr3[k] = w * r3;
-        }
-        const float pxy2 = 2.f * m.pxy, pxz2 = 2.f * m.pxz, pyz2 = 2.f * m.pyz;
-#pragma unroll
-        for (int i = 1; i < Q; i += 2) {
-            const int cx = lat_cx(i), cy = lat_cy(i), cz = lat_cz(i);
-            const int k = lat_norm1(i) - 1;   // 0 axis, 1 face diagonal, 2 body diagonal
-            float S = 0.f, cu = 0.f, cF = 0.f;
-            if (cx) { S += m.pxx; cu += cx * m.ux; cF += cx * fx; }
-            if (cy) { S += m.pyy; cu += cy * m.uy; cF += cy * fy; }
-            if (cz) { S += m.pzz; cu += cz * m.uz; cF += cz * fz; }
-            if (cx && cy) S += cx * cy * pxy2;
-            if (cx && cz) S += cx * cz * pxz2;
-            if (cy && cz) S += cy * cz * pyz2;
-            const float E = cK[k] + cA[k] * S + cu * (cr45[k] * cu + cb9[k] * cF);
-            const float O = cal[k] * cF + cr3[k] * cu;
-            f[i] = E + O;
-            f[i + 1] = E - O;
-        }
-    } else {
-        const float om1 = 1.f - omega;
-        // on deviations: (1 - omega) w rho0 + omega w rho0 cancels against w rho0
-        const float base = omega * (m.drho - 1.5f * m.rho * uu) - 3.f * B * uF;
-        const float r45 = 4.5f * omega * m.rho, r3 = 3.f * omega * m.rho, b9 = 9.f * B, b3 = 3.f * B;
-        f[0] = om1 * f[0] + Lattice<Q>::w(0) * base;
-#pragma unroll
-        for (int i = 1; i < Q; i += 2) {
-            const int cx = lat_cx(i), cy = lat_cy(i), cz = lat_cz(i);
-            float cu = 0.f, cF = 0.f;
-            if (cx) { cu += cx * m.ux; cF += cx * fx; }
-            if (cy) { cu += cy * m.uy; cF += cy * fy; }
-            if (cz) { cu += cz * m.uz; cF += cz * fz; }
-            const float w = Lattice<Q>::w(i);
-            const float E = w * (base + cu * (r45 * cu + b9 * cF));
-            const float O = w * (r3 * cu + b3 * cF);
-            f[i] = om1 * f[i] + (E + O);
-            f[i + 1] = om1 * f[i + 1] + (E - O);
-        }
-    }
 }
 
 // Everything after the gather for one node: IBM force read and reset
