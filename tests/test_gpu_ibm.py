@@ -178,3 +178,35 @@ def test_checkpoint_image_keeps_ibm_macroscopics_as_planes(vlbm):
     m = sim.macroscopics()
     for k, name in enumerate(("rho", "ux", "uy", "uz")):
         np.testing.assert_array_equal(planes[k][box], m[name][box])
+
+
+@pytest.mark.parametrize("diameter,iterations", [(3.0, 1), (8.0, 2), (11.0, 1)])
+def test_reading_nodes_between_steps_changes_nothing(vlbm, diameter, iterations):
+    """A step leaves its node movement to the next step's boxes; a reader takes
+    it at once, and the run goes on bit for bit as if nothing had been read."""
+    def make():
+        cfg = vlbm.Config.default(nx=24, ny=22, nz=20, tau=0.7, fx=1e-5)
+        sim = vlbm.Simulation(cfg, builder=vlbm.BUILDER_PLATES_Y)
+        sim.add_spheres(vlbm.IbmConfig.default(max_iterations=iterations),
+                        [vlbm.Sphere(diameter=diameter, cx=1.5, cy=10.5, cz=9.0, vx=-0.02, wy=0.01, density=2.0,
+                                     movable=1),
+                         vlbm.Sphere(diameter=4.0, cx=14.0, cy=11.0, cz=10.0, vz=0.01, density=2.0, movable=1)])
+        return sim
+    a, b = make(), make()
+    a.step(7)
+    for k in range(7):
+        b.step(1)
+        if k % 2 == 0:
+            b.lagrangian_nodes()
+            b.lagrangian_nodes()
+        if k == 3:
+            c = make()
+            c.restore(b.checkpoint())
+            b = c
+    for x, y in zip(a.lagrangian_nodes(), b.lagrangian_nodes()):
+        np.testing.assert_array_equal(x, y)
+    ma, mb = a.macroscopics(), b.macroscopics()
+    for k in ma:
+        np.testing.assert_array_equal(ma[k], mb[k])
+    for p, q in zip(a.particles(2), b.particles(2)):
+        assert list(p.pos) == list(q.pos) and list(p.vel) == list(q.vel) and list(p.w) == list(q.w)

@@ -523,12 +523,10 @@ vlbm_status vlbm_step(vlbm_sim* s, uint32_t nsteps) {
     CHECK_SIM(s);
     if (!s->geometry) { set_last_error("vlbm_set_node_map must be called before vlbm_step"); return VLBM_ERR_STATE; }
     for (uint32_t k = 0; k < nsteps; ++k) {
-        vlbm_status st = fluid_step(s);
+        vlbm_status st = s->ibm ? ibm_begin(s) : VLBM_OK;
+        if (st == VLBM_OK) st = fluid_step(s);
+        if (st == VLBM_OK && s->ibm) st = ibm_step(s);
         if (st != VLBM_OK) return st;
-        if (s->ibm) {
-            st = ibm_step(s);
-            if (st != VLBM_OK) return st;
-        }
     }
     return VLBM_OK;
 }

@@ -181,6 +181,7 @@ vlbm_status ready(vlbm_sim* s) {
     if (!s) { set_last_error("null simulation handle"); return VLBM_ERR_INVALID; }
     if (!s->geometry) { set_last_error("checkpoint: the simulation has no geometry yet"); return VLBM_ERR_STATE; }
     cudaError_t e = cudaSetDevice(s->device);
+    if (e == cudaSuccess) e = ibm_flush_nodes(s);   // the image holds moved nodes, and a loaded state has none to move
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
     return cuda_status(e, "checkpoint: synchronise");
 }

@@ -379,7 +379,7 @@ vlbm_status server_rebuild(vlbm_server* sv) {
         for (size_t i = 0; i < sv->res.size(); ++i) {
             const vlbm_sim* s = sv->res[i].sim;
             gpu_us += 2.0 * s->Q * s->store_bytes * (double)s->N / 4.5e6;
-            if (s->ibm) { host_us += 4.0 * (3.0 + 3.0 * std::max(1, ibm_iterations(s))); continue; }
+            if (s->ibm) { host_us += 4.0 * (4.0 + 2.0 * std::max(1, ibm_iterations(s))); continue; }
             const long long wave = sv->own_launch_min_nodes >= 0
                                        ? sv->own_launch_min_nodes
                                        : (long long)std::max(1, batched_blocks_per_sm(s->Q, s->cfg.storage,
@@ -575,7 +575,7 @@ vlbm_status server_rebuild(vlbm_server* sv) {
         double bytes = 0.0;
         for (const Resident& r : sv->res) {
             bytes += 2.0 * r.sim->Q * r.sim->store_bytes * (double)r.sim->N;
-            if (r.sim->ibm) launches += 3.0 + 3.0 * std::max(1, ibm_iterations(r.sim));
+            if (r.sim->ibm) launches += 4.0 + 2.0 * std::max(1, ibm_iterations(r.sim));
         }
         const double host_us = 4.0 * launches, gpu_us = bytes / 4.0e6;
         sv->use_graphs = gpu_us < 3.0 * host_us;
@@ -635,10 +635,11 @@ vlbm_status enqueue_steps(vlbm_server* sv, int n) {
         s->stream = side;
         vlbm_status st = VLBM_OK;
         for (int i = 0; i < n && st == VLBM_OK; ++i) {
-            st = fluid_step(s);   // advances the mirror
+            if (s->ibm) st = ibm_begin(s);
+            if (st == VLBM_OK) st = fluid_step(s);   // advances the mirror
             if (st == VLBM_OK && s->ibm) st = ibm_step(s);
         }
-        launches += (double)n * (1.0 + (s->ibm ? 2.0 + 3.0 * std::max(1, ibm_iterations(s)) : 0.0));
+        launches += (double)n * (1.0 + (s->ibm ? 3.0 + 2.0 * std::max(1, ibm_iterations(s)) : 0.0));
         s->stream = sv->stream;
         if (st != VLBM_OK) return st;
         e = cudaEventRecord(sv->join_events[j], side);
