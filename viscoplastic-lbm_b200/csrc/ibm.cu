@@ -290,7 +290,7 @@ __device__ __forceinline__ void gather_box_node(const StepParams& sp, const IbmP
     float f[Q];
     uint8_t cls;
     gather_node<Q, ST, ODD, PAIRED>(sp, n, nb, x, y, z, f, cls);
-    const Mom m = moments<Q, false>(f, P.fx, P.fy, P.fz, sp.rho0);
+    const Mom m = moments_st<ST, Q, false>(f, P.fx, P.fy, P.fz, sp.rho0);
     fields[n] = make_float4(m.rho, m.ux, m.uy, m.uz);
     atomicMin(&owner[n], sphere);
 }

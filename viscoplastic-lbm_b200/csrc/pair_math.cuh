@@ -1,5 +1,5 @@
-// pair_math.cuh -- the fused step's arithmetic, for one node (float) or for two
-// at once (float2).
+// pair_math.cuh -- the arithmetic of the half-precision step, for one node
+// (float) or for two at once (float2).  (FP32 storage: step_math_f32.cuh.)
 //
 // The z-paired kernel (k_step2) holds the nodes (x, y, z) and (x, y, z + NZ/2)
 // in the two lanes of float2 values and evaluates moments, stress magnitude
@@ -31,10 +31,12 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 rcp2(float2 a) { return make_float2(__frcp_rn(a.x), __frcp_rn(a.y)); }
-__device__ __forceinline__ float add2(float a, float b) { return a + b; }
-__device__ __forceinline__ float sub2(float a, float b) { return a - b; }
-__device__ __forceinline__ float mul2(float a, float b) { return a * b; }
-__device__ __forceinline__ float fma2(float a, float b, float c) { return fmaf(a, b, c); }
+// One node: the same roundings as a lane of the packed operations (no
+// contraction).
+__device__ __forceinline__ float add2(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float sub2(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ float mul2(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float fma2(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ float rcp2(float a) { return __frcp_rn(a); }
 template <class F> __device__ __forceinline__ F vs(float a);   // a in every lane
 template <> __device__ __forceinline__ float vs<float>(float a) { return a; }
@@ -195,7 +197,8 @@ __device__ __forceinline__ float2 stress_aux2(const Mom2& m, float2 fx, float2 f
 // sign at all nodes and steps: it acts as a force along the momentum.  So the
 // constants 3 w and 1/3 are products with their exact value (a second term
 // carries what rounding the constant leaves), and the half force enters V as F
-// minus what rounding j + F/2 has added already.  Against 64 bits, a Bingham
+// minus what rounding j + F/2 has added already (BGK: omega h + omega (F -
+// (h - j)) + (1 - omega) F, which is omega rho u + B F).  Against 64 bits, a Bingham
 // channel of 128 nodes at u = 0.07 after 50,000 steps (velocity, relative): D3Q19
 // 1.3e-4 - 1.6e-4 (0.9e-4 - 4.4e-4 with the formula evaluated per population),
 // D3Q27 1.4e-5 - 6e-5 (5e-4 - 9e-4).
@@ -213,35 +216,44 @@ __device__ __forceinline__ void collide_of(F (&g)[Q], const MomT<F>& m, F omega,
     const float w = Lattice<Q>::w(7) * oscale;
     constexpr float W3 = (float)(3.0 * Lattice<Q>::wd(7)), W3LO = (float)(3.0 * Lattice<Q>::wd(7) - (double)W3);
     const F w3 = vs<F>(W3 * oscale), w3lo = vs<F>(W3LO * oscale);
-    F Vx, Vy, Vz, cq, A, A2, om1;
+    F Vx, Vy, Vz, cq, A, A2, om1 = vs<F>(0.f);
+    // F minus the half force as it was rounded into h
+    const F ex = sub2(fx, sub2(m.hx, m.jx)), ey = sub2(fy, sub2(m.hy, m.jy)), ez = sub2(fz, sub2(m.hz, m.jz));
     if constexpr (REG) {
-        const F ex = sub2(fx, sub2(m.hx, m.jx)), ey = sub2(fy, sub2(m.hy, m.jy)), ez = sub2(fz, sub2(m.hz, m.jz));
         Vx = fma2(m.hx, w3, fma2(ex, w3, mul2(m.hx, w3lo)));
         Vy = fma2(m.hy, w3, fma2(ey, w3, mul2(m.hy, w3lo)));
         Vz = fma2(m.hz, w3, fma2(ez, w3, mul2(m.hz, w3lo)));
         cq = fma2(omega, vs<F>(-4.5f * w), vs<F>(6.75f * w));
         A = fma2(omega, vs<F>(-4.5f * w), vs<F>(4.5f * w));
         A2 = add2(A, A);
-    } else {
-        const F B3 = fma2(omega, vs<F>(-1.5f * w), vs<F>(3.f * w));
+    } else {   // omega h + omega e + (1 - omega) F
         const F hx = mul2(omega, m.hx), hy = mul2(omega, m.hy), hz = mul2(omega, m.hz);
-        Vx = fma2(hx, w3, fma2(fx, B3, mul2(hx, w3lo)));
-        Vy = fma2(hy, w3, fma2(fy, B3, mul2(hy, w3lo)));
-        Vz = fma2(hz, w3, fma2(fz, B3, mul2(hz, w3lo)));
-        cq = mul2(B3, vs<F>(1.5f));
+        const F ow = mul2(omega, w3), fw = fma2(omega, vs<F>(-W3 * oscale), w3);
+        Vx = fma2(hx, w3, fma2(ex, ow, fma2(fx, fw, mul2(hx, w3lo))));
+        Vy = fma2(hy, w3, fma2(ey, ow, fma2(fy, fw, mul2(hy, w3lo))));
+        Vz = fma2(hz, w3, fma2(ez, ow, fma2(fz, fw, mul2(hz, w3lo))));
+        cq = fma2(omega, vs<F>(-2.25f * w), vs<F>(4.5f * w));
         om1 = mul2(sub2(vs<F>(1.f), omega), vs<F>(gscale * oscale));
     }
     const F c15 = vs<F>(1.5f);
     const F qx = fma2(Vx, c15, mul2(cq, fx)), qy = fma2(Vy, c15, mul2(cq, fy)), qz = fma2(Vz, c15, mul2(cq, fz));
-    F Txx = mul2(m.ux, qx), Tyy = mul2(m.uy, qy), Tzz = mul2(m.uz, qz);
     F Txy = mul2(m.uy, qx), Txz = mul2(m.uz, qx), Tyz = mul2(m.uz, qy);
+    F Txx, Tyy, Tzz;
     if constexpr (REG) {
-        Txx = fma2(A, m.pxx, Txx); Tyy = fma2(A, m.pyy, Tyy); Tzz = fma2(A, m.pzz, Tzz);
+        Txx = fma2(A, m.pxx, mul2(m.ux, qx)); Tyy = fma2(A, m.pyy, mul2(m.uy, qy));
+        Tzz = fma2(A, m.pzz, mul2(m.uz, qz));
         Txy = fma2(A2, m.pxy, Txy); Txz = fma2(A2, m.pxz, Txz); Tyz = fma2(A2, m.pyz, Tyz);
     }
+    // v + T_aa.  BGK's T_aa is a bare product: the sum is written as a fused
+    // operation, because the compiler may fuse a packed product and sum by itself
+    auto plus_t = [&](F v, int a) {
+        if constexpr (REG) return add2(v, a == 0 ? Txx : (a == 1 ? Tyy : Tzz));
+        else return a == 0 ? fma2(m.ux, qx, v) : (a == 1 ? fma2(m.uy, qy, v) : fma2(m.uz, qz, v));
+    };
     Txy = fma2(m.ux, qy, Txy); Txz = fma2(m.ux, qz, Txz); Tyz = fma2(m.uy, qz, Tyz);
     constexpr float T3 = -1.f / 3.f, T3LO = (float)(-1.0 / 3.0 - (double)T3);
-    const F tr = add2(add2(Txx, Tyy), Tzz);
+    if constexpr (!REG) Txx = mul2(m.ux, qx);
+    const F tr = plus_t(plus_t(Txx, 1), 2);
     const F K = fma2(tr, vs<F>(T3), fma2(tr, vs<F>(T3LO), mul2(REG ? m.drho : mul2(omega, m.drho), vs<F>(w))));
     if constexpr (REG) g[0] = mul2(K, vs<F>(REST));
     else g[0] = fma2(om1, g[0], mul2(K, vs<F>(REST)));
@@ -255,12 +267,12 @@ __device__ __forceinline__ void collide_of(F (&g)[Q], const MomT<F>& m, F omega,
             g[i + 1] = fma2(om1, g[i + 1], sub2(E, O));
         }
     };
-    const F Kx = add2(K, Txx), Ky = add2(K, Tyy), Kz = add2(K, Tzz);
+    const F Kx = plus_t(K, 0), Ky = plus_t(K, 1), Kz = plus_t(K, 2);
     const F ax = vs<F>(AXIS);
     put(1, mul2(Kx, ax), mul2(Vx, ax));
     put(3, mul2(Ky, ax), mul2(Vy, ax));
     put(5, mul2(Kz, ax), mul2(Vz, ax));
-    const F Exy = add2(Kx, Tyy), Exz = add2(Kx, Tzz), Eyz = add2(Ky, Tzz);
+    const F Exy = plus_t(Kx, 1), Exz = plus_t(Kx, 2), Eyz = plus_t(Ky, 2);
     const F Vp = add2(Vx, Vy), Vm = sub2(Vx, Vy);
     put(7, add2(Exy, Txy), Vp);
     put(13, sub2(Exy, Txy), Vm);
@@ -270,7 +282,7 @@ __device__ __forceinline__ void collide_of(F (&g)[Q], const MomT<F>& m, F omega,
     put(17, sub2(Eyz, Tyz), sub2(Vy, Vz));
     if constexpr (Q == 27) {
         const F bd = vs<F>(BODY);
-        const F E = mul2(add2(Exy, Tzz), bd), Sxy = mul2(Txy, bd);
+        const F E = mul2(plus_t(Exy, 2), bd), Sxy = mul2(Txy, bd);
         const F p = mul2(add2(Txz, Tyz), bd), q = mul2(sub2(Txz, Tyz), bd);
         const F b1 = add2(E, Sxy), b2 = sub2(E, Sxy);
         const F vp = mul2(Vp, bd), vm = mul2(Vm, bd), vz = mul2(Vz, bd);

@@ -30,6 +30,7 @@
 #include "internal.h"
 #include "lattice.cuh"
 #include "pair_math.cuh"
+#include "step_math_f32.cuh"
 
 namespace vlbm {
 
@@ -516,7 +517,7 @@ __device__ __forceinline__ float relax(const StepParams& p, float eta_old, float
 // (lbm.cu:45-58), moments, relaxation (lbm.cu:192-222), collision, and the
 // post-collision copy of boundary nodes (lbm.cu:463-470).  `eta_old` is the
 // node's Power-Law state p.omega[n], loaded by the caller ahead of the gather.
-template <int Q, int OP, int RHEO>
+template <int ST, int Q, int OP, int RHEO>
 __device__ __forceinline__ void relax_and_collide(const StepParams& p, float* side_next, unsigned n, uint8_t cls,
                                                   int slot, float (&f)[Q], float eta_old) {
     float fx = p.fx, fy = p.fy, fz = p.fz;
@@ -527,16 +528,16 @@ __device__ __forceinline__ void relax_and_collide(const StepParams& p, float* si
         p.cls[n] = cls & (uint8_t)~NODE_IBM_FORCE;
     }
     constexpr bool NEED_PI = (OP == VLBM_OP_REGULARIZED) || (RHEO != VLBM_NEWTONIAN);
-    const Mom m = moments<Q, NEED_PI>(f, fx, fy, fz, p.rho0);
+    const Mom m = moments_st<ST, Q, NEED_PI>(f, fx, fy, fz, p.rho0);
     if (!(m.rho > 0.f && m.rho < 1e30f) && !(cls & NODE_UNUSED)) atomicOr(p.err, 1u);
     float omega = p.omega_newt;
     if (RHEO != VLBM_NEWTONIAN) {
-        const float aux = stress_aux(m, fx, fy, fz);
+        const float aux = stress_aux_st<ST>(m, fx, fy, fz);
         float eta = 0.f;
         omega = relax<RHEO>(p, eta_old, aux, eta);
         if (RHEO == VLBM_POWERLAW) p.omega[n] = eta;  // state update, lbm.cu:215-219
     }
-    collide<Q, OP>(f, m, omega, fx, fy, fz);
+    collide_st<ST, Q, OP>(f, m, omega, fx, fy, fz);
     if (cls & NODE_UNUSED) {   // lbm.cu:23-24: not updated; rest equilibrium stays in its slots
 #pragma unroll
         for (int i = 0; i < Q; ++i) f[i] = 0.f;
@@ -547,12 +548,6 @@ __device__ __forceinline__ void relax_and_collide(const StepParams& p, float* si
         for (int i = 0; i < Q; ++i) side_next[(size_t)i * nbc + slot] = f[i];
     }
 }
-template <int Q, int OP, int RHEO>
-__device__ __forceinline__ void relax_and_collide(const StepParams& p, unsigned n, uint8_t cls, int slot,
-                                                  float (&f)[Q]) {
-    relax_and_collide<Q, OP, RHEO>(p, p.side_next, n, cls, slot, f, (RHEO == VLBM_POWERLAW) ? p.omega[n] : 0.f);
-}
-
 // ------------------------------------------------------------ kernels --
 // Occupancy: the odd (neighbour) step needs more address registers; capping it
 // at 4 resident 256-thread blocks per SM (64 registers) keeps enough loads in
@@ -573,7 +568,7 @@ __device__ __forceinline__ void step_node(const StepParams& p, const float* side
     float f[Q];
     uint8_t cls;
     const int slot = gather<Q, ST, ODD>(p, side_prev, use_bc, n, nb, x, y, z, f, cls);
-    relax_and_collide<Q, OP, RHEO>(p, side_next, n, cls, slot, f, eta_old);
+    relax_and_collide<ST, Q, OP, RHEO>(p, side_next, n, cls, slot, f, eta_old);
     nb.launder();
     Rng rng(n, seed);
     T* plane = static_cast<T*>(p.pop);
@@ -730,7 +725,7 @@ __global__ void __launch_bounds__(256) k_macro(const MacroParams mp) {
         return;
     }
     constexpr bool NEED_PI = RHEO != VLBM_NEWTONIAN;
-    const Mom m = moments<Q, NEED_PI>(f, fx, fy, fz, p.rho0);
+    const Mom m = moments_st<ST, Q, NEED_PI>(f, fx, fy, fz, p.rho0);
     if (mp.rho) mp.rho[n] = m.rho;
     if (mp.ux) mp.ux[n] = m.ux;
     if (mp.uy) mp.uy[n] = m.uy;
@@ -738,7 +733,7 @@ __global__ void __launch_bounds__(256) k_macro(const MacroParams mp) {
     if (mp.omega_out) {
         float omega = p.omega_newt;
         if (RHEO != VLBM_NEWTONIAN) {
-            const float aux = stress_aux(m, fx, fy, fz);
+            const float aux = stress_aux_st<ST>(m, fx, fy, fz);
             const float old = (RHEO == VLBM_POWERLAW) ? p.omega[n] : 0.f;
             float eta = 0.f;
             omega = relax<RHEO>(p, old, aux, eta);
@@ -1076,13 +1071,13 @@ __device__ __forceinline__ void step2_pair(const StepParams& p, const unsigned s
         }
     }
     constexpr bool NEED_PI = (OP == VLBM_OP_REGULARIZED) || (RHEO != VLBM_NEWTONIAN);
-    const Mom2 mm = moments2<Q, NEED_PI, SC>(g, fx2, fy2, fz2, p.rho0, p.inv_scale);
+    const Mom2 mm = moments2_st<ST, Q, NEED_PI, SC>(g, fx2, fy2, fz2, p.rho0, p.inv_scale);
     if ((!(mm.rho.x > 0.f && mm.rho.x < 1e30f) && !(c0 & NODE_UNUSED)) ||
         (!(mm.rho.y > 0.f && mm.rho.y < 1e30f) && !(c1 & NODE_UNUSED)))
         atomicOr(p.err, 1u);
     float2 omega = f2(p.omega_newt);
     if (RHEO != VLBM_NEWTONIAN) {
-        const float2 aux = stress_aux2(mm, fx2, fy2, fz2);
+        const float2 aux = stress_aux2_st<ST>(mm, fx2, fy2, fz2);
 #pragma unroll
         for (int lane = 0; lane < 2; ++lane) {
             const unsigned nl = lane ? n1 : n0;
@@ -1092,7 +1087,7 @@ __device__ __forceinline__ void step2_pair(const StepParams& p, const unsigned s
         }
     }
     // post-collision values as stored: deviations times the storage scale
-    collide2<Q, OP>(g, mm, omega, fx2, fy2, fz2, SC ? p.inv_scale : 1.f, SC ? p.scale : 1.f);
+    collide2_st<ST, Q, OP>(g, mm, omega, fx2, fy2, fz2, SC ? p.inv_scale : 1.f, SC ? p.scale : 1.f);
     if (!BULK && ((c0 | c1) & NODE_UNUSED)) {   // lbm.cu:23-24: not updated; rest equilibrium stays in the slots
         const bool u0 = c0 & NODE_UNUSED, u1 = c1 & NODE_UNUSED;
 #pragma unroll
@@ -1216,8 +1211,8 @@ __global__ void __launch_bounds__(256, 2) k_macro2(const MacroParams mp) {
     if ((c0 | c1) & NODE_BC) pair_boundary<Q, ST>(p, pr.x, pr.y, pr.zp, nn[0], nn[1], c0, c1, g, s0, s1);
     constexpr bool NEED_PI = RHEO != VLBM_NEWTONIAN;
     const float2 fx2 = f2(p.fx), fy2 = f2(p.fy), fz2 = f2(p.fz);
-    const Mom2 mm = moments2<Q, NEED_PI, SC>(g, fx2, fy2, fz2, p.rho0, p.inv_scale);
-    const float2 aux = NEED_PI ? stress_aux2(mm, fx2, fy2, fz2) : f2(0.f);
+    const Mom2 mm = moments2_st<ST, Q, NEED_PI, SC>(g, fx2, fy2, fz2, p.rho0, p.inv_scale);
+    const float2 aux = NEED_PI ? stress_aux2_st<ST>(mm, fx2, fy2, fz2) : f2(0.f);
 #pragma unroll
     for (int lane = 0; lane < 2; ++lane) {
         const unsigned n = nn[lane];
