@@ -36,9 +36,13 @@ def test_paired_readout_equals_natural(size, q, rheo, st, builder):
         sim.set_layout(vlbm.LAYOUT_ZPAIR)
         # the interpolated rule is the only one with products: its sums may contract differently
         assert np.abs(pops - pops_n).max() <= (2e-7 if builder == vlbm.BUILDER_CIRCULAR_DUCT else 0.0)
-        # sums of Q deviations |g| <= 0.1 w and one reciprocal: 27 * 2^-24 * 0.1 and a few ulp of 1
-        for k in ("rho", "ux", "uy", "uz"):
-            assert np.abs(pair[k] - nat[k]).max() <= 1e-6, k
-        ok = np.abs(pair["omega"] - nat["omega"]) <= 1e-3 * np.abs(nat["omega"]) + 1e-4
-        assert ok.mean() > 0.995 and np.isfinite(pair["omega"]).all() == np.isfinite(nat["omega"]).all()
+        # the same operations in both read-outs, so the same bits; after the interpolated rule, sums of Q
+        # deviations |g| <= 0.1 w and one reciprocal: 27 * 2^-24 * 0.1 and a few ulp of 1
+        for k in pair:
+            if builder != vlbm.BUILDER_CIRCULAR_DUCT:
+                np.testing.assert_array_equal(pair[k], nat[k], err_msg=k)
+            else:
+                # omega follows the stress, whose 1e-7 is 1e-4 of the 1e-3 that these populations have
+                tol = 1e-3 * np.abs(nat[k]) + 1e-4 if k == "omega" else 1e-6
+                assert np.all(np.abs(pair[k] - nat[k]) <= tol), k
     sim.close()

@@ -1210,24 +1210,45 @@ __global__ void __launch_bounds__(256, 2) k_macro2(const MacroParams mp) {
     int s0 = -1, s1 = -1;
     if ((c0 | c1) & NODE_BC) pair_boundary<Q, ST>(p, pr.x, pr.y, pr.zp, nn[0], nn[1], c0, c1, g, s0, s1);
     constexpr bool NEED_PI = RHEO != VLBM_NEWTONIAN;
-    const float2 fx2 = f2(p.fx), fy2 = f2(p.fy), fz2 = f2(p.fz);
-    const Mom2 mm = moments2_st<ST, Q, NEED_PI, SC>(g, fx2, fy2, fz2, p.rho0, p.inv_scale);
-    const float2 aux = NEED_PI ? stress_aux2_st<ST>(mm, fx2, fy2, fz2) : f2(0.f);
+    Mom m2[2];
+    float aux[2];
+    if constexpr (ST == VLBM_STORE_F32) {   // by node: the packed sums round omega's stress differently
+#pragma unroll
+        for (int lane = 0; lane < 2; ++lane) {
+            float f[Q];
+#pragma unroll
+            for (int i = 0; i < Q; ++i) f[i] = lane_of(g[i], lane);
+            m2[lane] = moments_st<ST, Q, NEED_PI>(f, p.fx, p.fy, p.fz, p.rho0);
+            aux[lane] = NEED_PI ? stress_aux_st<ST>(m2[lane], p.fx, p.fy, p.fz) : 0.f;
+        }
+    } else {
+        const float2 fx2 = f2(p.fx), fy2 = f2(p.fy), fz2 = f2(p.fz);
+        const Mom2 mm = moments2_st<ST, Q, NEED_PI, SC>(g, fx2, fy2, fz2, p.rho0, p.inv_scale);
+        const float2 a2 = NEED_PI ? stress_aux2_st<ST>(mm, fx2, fy2, fz2) : f2(0.f);
+#pragma unroll
+        for (int lane = 0; lane < 2; ++lane) {
+            m2[lane].rho = lane_of(mm.rho, lane);
+            m2[lane].ux = lane_of(mm.ux, lane);
+            m2[lane].uy = lane_of(mm.uy, lane);
+            m2[lane].uz = lane_of(mm.uz, lane);
+            aux[lane] = lane_of(a2, lane);
+        }
+    }
 #pragma unroll
     for (int lane = 0; lane < 2; ++lane) {
         const unsigned n = nn[lane];
         // an unused node is never updated: the initial macroscopics (lbmInitialization.cu:100-111)
         const bool unused = (lane ? c1 : c0) & NODE_UNUSED;
-        if (mp.rho) mp.rho[n] = unused ? p.rho0 : lane_of(mm.rho, lane);
-        if (mp.ux) mp.ux[n] = unused ? 0.f : lane_of(mm.ux, lane);
-        if (mp.uy) mp.uy[n] = unused ? 0.f : lane_of(mm.uy, lane);
-        if (mp.uz) mp.uz[n] = unused ? 0.f : lane_of(mm.uz, lane);
+        if (mp.rho) mp.rho[n] = unused ? p.rho0 : m2[lane].rho;
+        if (mp.ux) mp.ux[n] = unused ? 0.f : m2[lane].ux;
+        if (mp.uy) mp.uy[n] = unused ? 0.f : m2[lane].uy;
+        if (mp.uz) mp.uz[n] = unused ? 0.f : m2[lane].uz;
         if (mp.omega_out) {
             float omega = p.omega_newt;
             if (RHEO != VLBM_NEWTONIAN) {
                 const float old = (RHEO == VLBM_POWERLAW) ? p.omega[n] : 0.f;
                 float eta = 0.f;
-                omega = relax<RHEO>(p, old, lane_of(aux, lane), eta);
+                omega = relax<RHEO>(p, old, aux[lane], eta);
             }
             mp.omega_out[n] = unused ? 0.f : omega;
         }
