@@ -144,3 +144,35 @@ def test_rejected_images_leave_the_simulation_unchanged(vlbm):
                                          ctypes.byref(need))
     assert st == vlbm.ERR_INVALID and need.value == image.size
     assert not small.any()
+
+
+def _pool_high(reset=False):
+    """Bytes that the device's default memory pool (cudaMallocAsync) has lent out at most since the last reset."""
+    cu = ctypes.CDLL("libcuda.so.1")
+    pool, value = ctypes.c_void_p(), ctypes.c_uint64(0)
+    assert cu.cuDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+    high = 8   # CU_MEMPOOL_ATTR_USED_MEM_HIGH
+    if reset:
+        assert cu.cuMemPoolSetAttribute(pool, high, ctypes.byref(value)) == 0
+    assert cu.cuMemPoolGetAttribute(pool, high, ctypes.byref(value)) == 0
+    return value.value
+
+
+# node counts of the IBM records: one part-filled chunk, and a full chunk with a remainder
+@pytest.mark.parametrize("size", [(24, 20, 24), (72, 66, 60)], ids=lambda s: "x".join(map(str, s)))
+def test_sphere_checkpoint_needs_no_device_memory(vlbm, size):
+    """A lattice that fills the device can be saved, and a load cannot run out
+    of device memory half way through the state."""
+    nx, ny, nz = size
+    cfg_kw = dict(nx=nx, ny=ny, nz=nz, vel_set=19, tau=0.7)
+    a, b = make(vlbm, cfg_kw, 3, SPHERES), make(vlbm, cfg_kw, 3, SPHERES)
+    a.step(3)
+    a.sync()
+    before, free = _pool_high(reset=True), a.info().device_bytes
+    image = a.checkpoint()
+    b.restore(image)
+    assert _pool_high() == before and a.info().device_bytes == free
+    np.testing.assert_array_equal(b.checkpoint(), image)
+    a.step(4)
+    b.step(4)
+    assert_same(state(b, SPHERES), state(a, SPHERES))

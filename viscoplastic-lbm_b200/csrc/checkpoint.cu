@@ -28,8 +28,11 @@
 // The file form is PATH/ID/checkpoint/0_state.bin, with '/' separators on
 // every platform (the reference's save path joins with "\\\\" on Linux).
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <memory>
+#include <new>
 #include <string>
 #include <sys/stat.h>
 #include <vector>
@@ -89,26 +92,57 @@ cudaError_t ckpt_copy(vlbm_sim* s, void* dst, const void* src, size_t bytes, cud
     return e == cudaSuccess ? cudaStreamSynchronize(s->stream) : e;
 }
 
-// One region between the device and the image (to_image: out of the device).
-// A region of float4 records goes through planes on the device, so the image
-// does not depend on how the device lays the four values out.
-cudaError_t region_copy(vlbm_sim* s, const StateRegion& r, void* host, bool to_image) {
-    if (!r.records4)
-        return to_image ? ckpt_copy(s, host, r.dev, r.bytes, cudaMemcpyDeviceToHost)
-                        : ckpt_copy(s, r.dev, host, r.bytes, cudaMemcpyHostToDevice);
-    const size_t N = r.bytes / (4 * sizeof(float));
-    void* planes = nullptr;
-    cudaError_t e = cudaMallocAsync(&planes, r.bytes, s->stream);
-    if (e != cudaSuccess) return e;
-    if (to_image) {
-        e = ibm_planes(r.dev, static_cast<float*>(planes), N, true, s->stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(host, planes, r.bytes, cudaMemcpyDeviceToHost, s->stream);
-    } else {
-        e = cudaMemcpyAsync(planes, host, r.bytes, cudaMemcpyHostToDevice, s->stream);
-        if (e == cudaSuccess) e = ibm_planes(r.dev, static_cast<float*>(planes), N, false, s->stream);
+// Host buffer through which a region of float4 records passes, in nodes (4 MB).
+constexpr size_t kRecordChunk = (size_t)1 << 18;
+struct Float4Chunk {
+    std::unique_ptr<float[]> buf;
+    // Room for the regions' records, if any has them; false: out of memory.
+    bool reserve(const std::vector<StateRegion>& regions) {
+        size_t nodes = 0;
+        for (const auto& r : regions)
+            if (r.records4) nodes = std::max(nodes, std::min(kRecordChunk, r.bytes / (4 * sizeof(float))));
+        if (nodes) buf.reset(new (std::nothrow) float[4 * nodes]);
+        return nodes == 0 || buf != nullptr;
     }
-    cudaFreeAsync(planes, s->stream);
-    return e == cudaSuccess ? cudaStreamSynchronize(s->stream) : e;
+};
+
+// One region between the device and the image (to_image: out of the device).
+// A region of float4 records is turned into planes on the host, chunk by chunk,
+// so the image does not depend on how the device lays the four values out and a
+// lattice that fills the device can still be saved and loaded.
+cudaError_t region_copy(vlbm_sim* s, const StateRegion& r, Float4Chunk& chunk, unsigned char* out,
+                        const unsigned char* in) {
+    const bool to_image = out != nullptr;
+    if (!r.records4)
+        return to_image ? ckpt_copy(s, out, r.dev, r.bytes, cudaMemcpyDeviceToHost)
+                        : ckpt_copy(s, r.dev, in, r.bytes, cudaMemcpyHostToDevice);
+    const size_t N = r.bytes / (4 * sizeof(float));
+    float* rec = chunk.buf.get();
+    for (size_t n0 = 0; n0 < N; n0 += kRecordChunk) {
+        const size_t n = std::min(kRecordChunk, N - n0), bytes = n * 4 * sizeof(float);
+        float* dev = static_cast<float*>(r.dev) + 4 * n0;
+        if (to_image) {
+            const cudaError_t e = ckpt_copy(s, rec, dev, bytes, cudaMemcpyDeviceToHost);
+            if (e != cudaSuccess) return e;
+        }
+        for (int c = 0; c < 4; ++c) {   // the image is not aligned for floats
+            const size_t plane = ((size_t)c * N + n0) * sizeof(float);
+            if (to_image)
+                for (size_t k = 0; k < n; ++k) std::memcpy(out + plane + 4 * k, rec + 4 * k + c, sizeof(float));
+            else
+                for (size_t k = 0; k < n; ++k) std::memcpy(rec + 4 * k + c, in + plane + 4 * k, sizeof(float));
+        }
+        if (!to_image) {
+            const cudaError_t e = ckpt_copy(s, dev, rec, bytes, cudaMemcpyHostToDevice);
+            if (e != cudaSuccess) return e;
+        }
+    }
+    return cudaSuccess;
+}
+
+vlbm_status out_of_host_memory() {
+    set_last_error("checkpoint: out of host memory");
+    return VLBM_ERR_NOMEM;
 }
 
 float effective_scale(const vlbm_sim* s) {
@@ -210,6 +244,8 @@ vlbm_status save_image(vlbm_sim* s, std::vector<unsigned char>* grow, void* buf,
             return VLBM_ERR_INVALID;
         }
     }
+    Float4Chunk chunk;
+    if (!chunk.reserve(regions)) return out_of_host_memory();
     size_t off = 0;
     std::memcpy(out, &h, sizeof(h));
     off += sizeof(h);
@@ -217,7 +253,7 @@ vlbm_status save_image(vlbm_sim* s, std::vector<unsigned char>* grow, void* buf,
         RegionHeader rh{r.id, 0u, (uint64_t)r.bytes};
         std::memcpy(out + off, &rh, sizeof(rh));
         off += sizeof(rh);
-        e = region_copy(s, r, out + off, true);
+        e = region_copy(s, r, chunk, out + off, nullptr);
         if (e != cudaSuccess) return cuda_status(e, "checkpoint: read device state");
         off += r.bytes;
     }
@@ -277,10 +313,12 @@ vlbm_status load_image(vlbm_sim* s, const unsigned char* in, size_t n) {
         if (rh.id != r.id || rh.bytes != r.bytes) return mismatch("state array " + std::to_string(r.id));
         off += sizeof(rh) + r.bytes;
     }
+    Float4Chunk chunk;   // before anything is written
+    if (!chunk.reserve(regions)) return out_of_host_memory();
     off = sizeof(CkptHeader);
     for (const auto& r : regions) {
         off += sizeof(RegionHeader);
-        cudaError_t e = region_copy(s, r, const_cast<unsigned char*>(in + off), false);
+        cudaError_t e = region_copy(s, r, chunk, nullptr, in + off);
         if (e != cudaSuccess) return cuda_status(e, "checkpoint: write device state");
         off += r.bytes;
     }

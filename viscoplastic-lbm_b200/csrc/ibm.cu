@@ -928,24 +928,6 @@ __global__ void __launch_bounds__(IBM_THREADS) k_ibm_fixup(IbmParams P, const DP
     }
 }
 
-// The IBM macroscopics as planes [4][N] (a checkpoint image keeps them so) from
-// the records, or back.
-__global__ void __launch_bounds__(IBM_THREADS) k_ibm_planes(float4* fields, float* planes, size_t N, int to_planes) {
-    const size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= N) return;
-    if (to_planes) {
-        const float4 m = fields[n];
-        planes[n] = m.x; planes[N + n] = m.y; planes[2 * N + n] = m.z; planes[3 * N + n] = m.w;
-    } else {
-        fields[n] = make_float4(planes[n], planes[N + n], planes[2 * N + n], planes[3 * N + n]);
-    }
-}
-cudaError_t ibm_planes(void* fields, float* planes, size_t N, bool to_planes, cudaStream_t s) {
-    k_ibm_planes<<<(unsigned)((N + IBM_THREADS - 1) / IBM_THREADS), IBM_THREADS, 0, s>>>(
-        static_cast<float4*>(fields), planes, N, to_planes ? 1 : 0);
-    return cudaGetLastError();
-}
-
 // ---------------------------------------------------------------- host --
 static void host_mesh(double diameter, double mesh_scale, double breugem, std::vector<double>& px,
                       std::vector<double>& py, std::vector<double>& pz, std::vector<double>& pS) {

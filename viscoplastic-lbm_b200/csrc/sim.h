@@ -130,8 +130,6 @@ struct StateRegion {
 // IBM hooks (ibm.cu)
 void ibm_state_regions(vlbm_sim* s, std::vector<StateRegion>& out);
 uint32_t ibm_record_bytes();   // bytes of one device particle record
-// float4 records of N nodes to planes [4][N] or back (device pointers).
-cudaError_t ibm_planes(void* fields, float* planes, size_t N, bool to_planes, cudaStream_t s);
 // One IBM step is ibm_begin, the fluid step, ibm_step.
 vlbm_status ibm_begin(vlbm_sim* s);
 vlbm_status ibm_step(vlbm_sim* s);
