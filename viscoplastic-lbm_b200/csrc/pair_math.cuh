@@ -196,12 +196,17 @@ __device__ __forceinline__ float2 stress_aux2(const Mom2& m, float2 fx, float2 f
 // A slow body-force flow (u / F ~ 1e4) shows every rounding that has the same
 // sign at all nodes and steps: it acts as a force along the momentum.  So the
 // constants 3 w and 1/3 are products with their exact value (a second term
-// carries what rounding the constant leaves), and the half force enters V as F
-// minus what rounding j + F/2 has added already (BGK: omega h + omega (F -
-// (h - j)) + (1 - omega) F, which is omega rho u + B F).  Against 64 bits, a Bingham
-// channel of 128 nodes at u = 0.07 after 50,000 steps (velocity, relative): D3Q19
-// 1.3e-4 - 1.6e-4 (0.9e-4 - 4.4e-4 with the formula evaluated per population),
-// D3Q27 1.4e-5 - 6e-5 (5e-4 - 9e-4).
+// carries what rounding the constant leaves).  The half force enters the
+// regularized V as F minus what rounding j + F/2 has added already, and drops
+// out of BGK's: omega rho u + B F = omega j + F.  FP16 storage, 256x128x64
+// Bingham channel after 50,000 steps, velocity against 64 bits at yield stresses
+// of 1.1e-6, 5.3e-6 and 4.7e-5: regularized D3Q19 1.7e-4, 1.7e-4, 1.7e-4 (7.2e-4,
+// 7.0e-4, 3.5e-4 with the formula evaluated per population), D3Q27 1.5e-4, 1.5e-4,
+// 1.6e-4 (7.2e-4, 6.9e-4, 3.5e-4); BGK D3Q19 1.3e-4, 2.3e-4 (7.6e-4, 6.9e-4) and
+// 5.9e-3 (5.7e-3) at the largest, where the plug hardly relaxes and keeps the
+// noise of the stores.  The D3Q19 one-node BGK step takes 21.4 us for Bingham and
+// 24.5 for Power-Law on 96x90x91 nodes, 21.5 and 25.3 with the half force in omega
+// h + omega (F - (h - j)) + (1 - omega) F.
 //
 // `gscale` is what the incoming g must be multiplied by to be deviations
 // (inv_scale for stored half values, 1 otherwise); the result is deviations
@@ -217,21 +222,21 @@ __device__ __forceinline__ void collide_of(F (&g)[Q], const MomT<F>& m, F omega,
     constexpr float W3 = (float)(3.0 * Lattice<Q>::wd(7)), W3LO = (float)(3.0 * Lattice<Q>::wd(7) - (double)W3);
     const F w3 = vs<F>(W3 * oscale), w3lo = vs<F>(W3LO * oscale);
     F Vx, Vy, Vz, cq, A, A2, om1 = vs<F>(0.f);
-    // F minus the half force as it was rounded into h
-    const F ex = sub2(fx, sub2(m.hx, m.jx)), ey = sub2(fy, sub2(m.hy, m.jy)), ez = sub2(fz, sub2(m.hz, m.jz));
     if constexpr (REG) {
+        // F minus the half force as it was rounded into h
+        const F ex = sub2(fx, sub2(m.hx, m.jx)), ey = sub2(fy, sub2(m.hy, m.jy)), ez = sub2(fz, sub2(m.hz, m.jz));
         Vx = fma2(m.hx, w3, fma2(ex, w3, mul2(m.hx, w3lo)));
         Vy = fma2(m.hy, w3, fma2(ey, w3, mul2(m.hy, w3lo)));
         Vz = fma2(m.hz, w3, fma2(ez, w3, mul2(m.hz, w3lo)));
         cq = fma2(omega, vs<F>(-4.5f * w), vs<F>(6.75f * w));
         A = fma2(omega, vs<F>(-4.5f * w), vs<F>(4.5f * w));
         A2 = add2(A, A);
-    } else {   // omega h + omega e + (1 - omega) F
-        const F hx = mul2(omega, m.hx), hy = mul2(omega, m.hy), hz = mul2(omega, m.hz);
-        const F ow = mul2(omega, w3), fw = fma2(omega, vs<F>(-W3 * oscale), w3);
-        Vx = fma2(hx, w3, fma2(ex, ow, fma2(fx, fw, mul2(hx, w3lo))));
-        Vy = fma2(hy, w3, fma2(ey, ow, fma2(fy, fw, mul2(hy, w3lo))));
-        Vz = fma2(hz, w3, fma2(ez, ow, fma2(fz, fw, mul2(hz, w3lo))));
+    } else {   // the half force drops out: omega rho u + B F = omega j + F
+        const F ow = mul2(omega, w3);
+        const F owlo = fma2(omega, w3lo, fma2(omega, w3, mul2(ow, vs<F>(-1.f))));   // what rounding 3 w omega leaves
+        Vx = fma2(m.jx, ow, fma2(fx, w3, mul2(m.jx, owlo)));
+        Vy = fma2(m.jy, ow, fma2(fy, w3, mul2(m.jy, owlo)));
+        Vz = fma2(m.jz, ow, fma2(fz, w3, mul2(m.jz, owlo)));
         cq = fma2(omega, vs<F>(-2.25f * w), vs<F>(4.5f * w));
         om1 = mul2(sub2(vs<F>(1.f), omega), vs<F>(gscale * oscale));
     }

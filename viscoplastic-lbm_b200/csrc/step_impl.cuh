@@ -605,8 +605,17 @@ __device__ __forceinline__ void step_chain_enter() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Resident 256-thread blocks per SM asked of the one-node kernel (0: the
+// compiler's choice of registers, 48 for D3Q19 and 64 for D3Q27).  D3Q27 BGK in
+// half storage keeps every population live through the collision and took 66 to
+// 74 registers, one block less: held to 64, 191x128x127 nodes take 95 us a step
+// against 103 for Bingham, 111 against 125 in a lid cavity.
+template <int Q, int OP, int ST> constexpr int step_blocks() {
+    return (ST != VLBM_STORE_F32 && Q == 27 && OP == VLBM_OP_BGK) ? 4 : 0;
+}
+
 template <int Q, int OP, int RHEO, int ST, bool ODD>
-__global__ void __launch_bounds__(256) k_step(const StepParams p) {
+__global__ void __launch_bounds__(256, step_blocks<Q, OP, ST>()) k_step(const StepParams p) {
     step_chain_enter();
     const unsigned seed = step_seed(p, ODD);
     const unsigned n = blockIdx.x * blockDim.x + threadIdx.x;
