@@ -39,6 +39,15 @@ def test_half_step_matches_oracle(oracle, q, op, rheo, storage, size):
     check_steps(oracle, q, op, rheo, storage, size)
 
 
+# the last lattice whose blocks are all resident at once (148 x 3 blocks of 256), and the first that is not
+@pytest.mark.parametrize("size", [(32, 32, 111), (41, 25, 111)], ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("storage", [vlbm.STORE_F16, vlbm.STORE_BF16])
+@pytest.mark.parametrize("rheo", [vlbm.NEWTONIAN, vlbm.BINGHAM])
+@pytest.mark.parametrize("op", [vlbm.OP_REGULARIZED, vlbm.OP_BGK])
+def test_half_step_matches_oracle_around_one_wave(oracle, op, rheo, storage, size):
+    check_steps(oracle, 27, op, rheo, storage, size)
+
+
 def check_steps(oracle, q, op, rheo, storage, size):
     nx, ny, nz = size
     cfg = vlbm.Config.default(nx=nx, ny=ny, nz=nz, vel_set=q, collision=op, rheology=rheo, storage=storage, tau=0.8,

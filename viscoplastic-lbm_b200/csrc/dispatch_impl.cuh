@@ -5,6 +5,8 @@
 
 namespace vlbm {
 
+constexpr int SMS = 148;   // B200
+
 inline unsigned grid_for(long long n, int block) { return (unsigned)((n + block - 1) / block); }
 
 // Launch that may start before the previous kernel of the stream has finished
@@ -58,8 +60,17 @@ cudaError_t step_t(const StepParams& p, bool odd, LaunchShape ls, cudaStream_t s
         return cudaGetLastError();
     }
     const unsigned g = grid_for(p.N, ls.block);   // chained to the previous step (step_chain_enter)
-    return odd ? launch_overlapped(k_step<Q, OP, RHEO, ST, true>, g, ls.block, s, p)
-               : launch_overlapped(k_step<Q, OP, RHEO, ST, false>, g, ls.block, s, p);
+    // one wave of the kernel with more registers: 32x76x45 (428 blocks) 5.7 us
+    // against 6.8, while 34x77x45 (461, two waves) in a lid cavity takes 9.1
+    // against 8.8 (D3Q27 FP16 Bingham)
+    constexpr int WIDE = step_blocks<Q, OP, ST, true>();
+    if constexpr (WIDE > 0) {
+        if (p.N <= (long long)SMS * 256 * WIDE)
+            return odd ? launch_overlapped(k_step<Q, OP, RHEO, ST, true, true>, g, ls.block, s, p)
+                       : launch_overlapped(k_step<Q, OP, RHEO, ST, false, true>, g, ls.block, s, p);
+    }
+    return odd ? launch_overlapped(k_step<Q, OP, RHEO, ST, true, false>, g, ls.block, s, p)
+               : launch_overlapped(k_step<Q, OP, RHEO, ST, false, false>, g, ls.block, s, p);
 }
 
 template <int Q, int OP, int ST>

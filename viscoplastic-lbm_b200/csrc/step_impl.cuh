@@ -606,16 +606,23 @@ __device__ __forceinline__ void step_chain_enter() {
 }
 
 // Resident 256-thread blocks per SM asked of the one-node kernel (0: the
-// compiler's choice of registers, 48 for D3Q19 and 64 for D3Q27).  D3Q27 BGK in
-// half storage keeps every population live through the collision and took 66 to
-// 74 registers, one block less: held to 64, 191x128x127 nodes take 95 us a step
-// against 103 for Bingham, 111 against 125 in a lid cavity.
-template <int Q, int OP, int ST> constexpr int step_blocks() {
-    return (ST != VLBM_STORE_F32 && Q == 27 && OP == VLBM_OP_BGK) ? 4 : 0;
+// compiler's choice of registers, 48 for D3Q19 and 64 for D3Q27).
+//
+// Half storage, D3Q27.  A lattice whose blocks are all resident at once has
+// nothing but its own loads to hide their latency: with three blocks (80
+// registers) they are all in flight, 32x76x45 nodes regularized Bingham 5.7 us a
+// step against 6.8 at 64 registers.  From the second wave on the fourth block is
+// worth more (step_t; 191x128x127: 92 us against 99, lid cavity 110 against 127).
+// BGK then has to be held to 64 registers: it keeps every population live through
+// the collision and took 66 to 74 (191x128x127: 95 us against 103, cavity 111
+// against 125).
+template <int Q, int OP, int ST, bool ONE_WAVE> constexpr int step_blocks() {
+    if (ST == VLBM_STORE_F32 || Q == 19) return 0;
+    return ONE_WAVE ? 3 : (OP == VLBM_OP_BGK ? 4 : 0);
 }
 
-template <int Q, int OP, int RHEO, int ST, bool ODD>
-__global__ void __launch_bounds__(256, step_blocks<Q, OP, ST>()) k_step(const StepParams p) {
+template <int Q, int OP, int RHEO, int ST, bool ODD, bool ONE_WAVE>
+__global__ void __launch_bounds__(256, step_blocks<Q, OP, ST, ONE_WAVE>()) k_step(const StepParams p) {
     step_chain_enter();
     const unsigned seed = step_seed(p, ODD);
     const unsigned n = blockIdx.x * blockDim.x + threadIdx.x;
