@@ -308,7 +308,6 @@ vlbm_status sim_macroscopics_device(vlbm_sim* s, float* rho, float* ux, float* u
     std::memset(&mp, 0, sizeof(mp));
     mp.s = make_params(s);
     mp.rho = rho; mp.ux = ux; mp.uy = uy; mp.uz = uz; mp.omega_out = omega;
-    mp.fibm_const = nullptr;
     cudaError_t e = launch_macro(s->Q, s->cfg.storage, mp, s->cfg.rheology, s->parity == 1, s->stream);
     if (e != cudaSuccess) return cuda_status(e, "macroscopics launch");
     if (s->ibm) return ibm_macroscopics_fixup(s, rho, ux, uy, uz);

@@ -143,19 +143,6 @@ __device__ __forceinline__ float stencil4(float x) {
     return 0.f;
 }
 
-__device__ __forceinline__ double block_sum(double v, double* sh) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) sh[warp] = v;
-    __syncthreads();
-    double s = 0.0;
-    if (threadIdx.x == 0)
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += sh[w];
-    return s;  // valid in thread 0
-}
-
 // gpuParticleNodeMovement ibm.cu:1044-1197
 __device__ void move_node(const IbmParams& P, const DMove& p, double* X, double* Y, double* Z, int k) {
     const double L[3] = {(double)P.nx, (double)P.ny, (double)P.nz};

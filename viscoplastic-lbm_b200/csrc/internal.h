@@ -85,7 +85,6 @@ struct StepParams {
 struct MacroParams {
     StepParams s;
     float *rho, *ux, *uy, *uz, *omega_out;
-    const float* fibm_const;    // IBM force to use in the half-force correction (may be null)
 };
 
 // Host-side analysis of a reference node map.

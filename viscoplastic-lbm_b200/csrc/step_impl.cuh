@@ -727,11 +727,6 @@ __global__ void __launch_bounds__(256) k_macro(const MacroParams mp) {
     float f[Q];
     uint8_t cls;
     gather<Q, ST, ODD>(p, n, nb, x, y, z, f, cls);
-    float fx = p.fx, fy = p.fy, fz = p.fz;
-    if (mp.fibm_const) {
-        const size_t N = (size_t)p.N;
-        fx += mp.fibm_const[n]; fy += mp.fibm_const[N + n]; fz += mp.fibm_const[2 * N + n];
-    }
     if (cls & NODE_UNUSED) {   // never updated: the initial macroscopics (lbmInitialization.cu:100-111)
         if (mp.rho) mp.rho[n] = p.rho0;
         if (mp.ux) mp.ux[n] = 0.f;
@@ -741,7 +736,7 @@ __global__ void __launch_bounds__(256) k_macro(const MacroParams mp) {
         return;
     }
     constexpr bool NEED_PI = RHEO != VLBM_NEWTONIAN;
-    const Mom m = moments_st<ST, Q, NEED_PI>(f, fx, fy, fz, p.rho0);
+    const Mom m = moments_st<ST, Q, NEED_PI>(f, p.fx, p.fy, p.fz, p.rho0);
     if (mp.rho) mp.rho[n] = m.rho;
     if (mp.ux) mp.ux[n] = m.ux;
     if (mp.uy) mp.uy[n] = m.uy;
@@ -749,7 +744,7 @@ __global__ void __launch_bounds__(256) k_macro(const MacroParams mp) {
     if (mp.omega_out) {
         float omega = p.omega_newt;
         if (RHEO != VLBM_NEWTONIAN) {
-            const float aux = stress_aux_st<ST>(m, fx, fy, fz);
+            const float aux = stress_aux_st<ST>(m, p.fx, p.fy, p.fz);
             const float old = (RHEO == VLBM_POWERLAW) ? p.omega[n] : 0.f;
             float eta = 0.f;
             omega = relax<RHEO>(p, old, aux, eta);
