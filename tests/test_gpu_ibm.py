@@ -139,6 +139,7 @@ def test_ibm_step_bit_reproducible(vlbm):
 @pytest.mark.parametrize("diameter,center,walls", [
     (1.5, (7.9, 8.2, 8.4), 1),      # few nodes: part-filled groups of lanes, one CTA
     (3.0, (0.4, 8.1, 9.0), 0),      # stencils across a periodic face
+    (3.0, (0.4, 8.1, 15.7), 0),     # stencils across two periodic faces
     (7.0, (8.3, 3.6, 8.0), 1),      # stencils cut by a wall
     (9.0, (8.1, 8.0, 7.8), 0),      # several CTAs per sphere, the last one part-filled
 ])
@@ -210,3 +211,36 @@ def test_reading_nodes_between_steps_changes_nothing(vlbm, diameter, iterations)
         np.testing.assert_array_equal(ma[k], mb[k])
     for p, q in zip(a.particles(2), b.particles(2)):
         assert list(p.pos) == list(q.pos) and list(p.vel) == list(q.vel) and list(p.w) == list(q.w)
+
+
+@pytest.mark.parametrize("storage", [0, 1, 2], ids=["f32", "f16", "bf16"])
+@pytest.mark.parametrize("q", [19, 27])
+@pytest.mark.parametrize("size", [(32, 20, 24), (20, 20, 24), (20, 20, 23)], ids=lambda s: "x".join(map(str, s)))
+def test_ibm_macroscopics_are_those_of_the_populations(vlbm, oracle, q, storage, size):
+    """rho and u of the sphere boxes come from the IBM step's own read of single
+    nodes (natural layout, node pairs, blocked pairs).  With the force that it
+    spread, they are the moments of the populations: rho = sum f, rho u = sum c f
+    + F / 2.  The spheres cross the plane where the pairs' lanes change (NZ / 2),
+    the periodic z seam and an x face.  Sums of Q values below 0.4 in FP32 and
+    one quotient: below 1e-6."""
+    nx, ny, nz = size
+    cfg = vlbm.Config.default(nx=nx, ny=ny, nz=nz, vel_set=q, storage=storage, tau=0.8, fx=1e-4,
+                              layout=vlbm.LAYOUT_NATURAL if nz % 2 else vlbm.LAYOUT_ZPAIR)
+    sim = vlbm.Simulation(cfg, builder=vlbm.BUILDER_PLATES_Y)
+    assert sim.info().layout == (0 if nz % 2 else 2 if nx % 32 == 0 else 1)
+    rng = np.random.default_rng(2)
+    sim.set_populations((sim.populations() * (1 + 0.02 * rng.standard_normal((q, nz, ny, nx)))).astype(np.float32))
+    sim.add_spheres(vlbm.IbmConfig.default(max_iterations=2, gx=0.0, gy=0.0, gz=-1e-5),
+                    [vlbm.Sphere(diameter=6.0, cx=8.2, cy=9.6, cz=nz / 2, vx=0.01, density=1.5, movable=1),
+                     vlbm.Sphere(diameter=5.0, cx=0.7, cy=9.4, cz=nz - 0.6, vz=0.01, density=1.5, movable=1)])
+    c = np.array(oracle.velocities(q), dtype=np.float64)
+    for step in (1, 2, 3):
+        sim.step(1)
+        m, f, force = sim.macroscopics(), sim.populations().astype(np.float64), sim.forces().astype(np.float64)
+        assert np.count_nonzero(force[2]) > 200          # the spread force reaches the nodes around both spheres
+        rho = f.sum(0)
+        assert np.abs(m["rho"] - rho).max() <= 1e-6, step
+        for a, name in enumerate(("ux", "uy", "uz")):
+            u = (np.tensordot(c[:, a], f, 1) + 0.5 * force[a]) / rho
+            assert np.abs(m[name] - u).max() <= 1e-6, (step, name)
+    sim.close()
