@@ -154,9 +154,9 @@ __device__ __forceinline__ Mom2 moments2(const float2 (&g)[Q], float2 fx, float2
     return moments_of<Q, NEED_PI, SCALED, float2>(g, fx, fy, fz, rho0, inv_scale);
 }
 
-// Twice the squared stress magnitude of the rheology models, with the force
-// correction (lbm.cu:192-208), and its square root: the hardware reciprocal
-// square root (<= 2 ulp).
+// The squared stress magnitude |S|^2 = S_ab S_ab / 2 of the rheology models, with
+// the force correction (lbm.cu:192-208), and its square root: the hardware
+// reciprocal square root (<= 2 ulp).
 template <class F>
 __device__ __forceinline__ F stress_square(const MomT<F>& m, F fx, F fy, F fz) {
     const F a = fma2(m.ux, fx, m.pxx), b = fma2(m.uy, fy, m.pyy), c = fma2(m.uz, fz, m.pzz);
